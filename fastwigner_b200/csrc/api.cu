@@ -100,7 +100,7 @@ extern "C" int fw_wigner_plan_create(int P, int X, int batch, int dtype, fw_wign
                                std::to_string(P) + " x " + std::to_string(X) + ")");
   if (batch < 1 || batch > 65535) return fail(FW_EINVAL, "fw_wigner_plan_create: batch must be in [1, 65535]");
   const int small = small_shapes(dtype, P, X, batch);
-  const int np = col_parts(dtype, P, X, small);
+  const int np = col_parts(dtype, P, X, small, batch);
   if (np <= 0) return fail(FW_EINVAL, "fw_wigner_plan_create: unsupported X for the column pass tile");
   fw_wigner_plan* p = new fw_wigner_plan();
   p->P = P; p->X = X; p->batch = batch; p->dtype = dtype; p->nparts = np; p->small = small;
@@ -288,9 +288,9 @@ extern "C" int fw_wigner_propagate(fw_wigner_plan* plan, const fw_wigner_desc* d
   if (d->step_kind == FW_STEP_FUSED) {
     // The two potential half-steps between kinetic steps share one transform
     // pair (observables from the mid-point spectrum) unless an x-p mask
-    // (bxp) sits between them, or the p-weights change with the step or do
-    // not fit the plan's spectrum buffer.
-    bool fuse = d->bxp == nullptr && !col_generic(plan->dtype, plan->P, plan->X);
+    // (bxp) sits between them, the p-weights change with the step or do not
+    // fit the plan's spectrum buffer, or an FP32 transform has a large prime.
+    bool fuse = d->bxp == nullptr && gen_fuses(plan->dtype, plan->P);
     if (fuse && d->Mp > 0) {
       const int nb = d->wp_bstride != 0 ? B : 1;
       if (d->wp_step != 0 || plan->wph == nullptr || nb > plan->wph_nb) {
@@ -510,7 +510,7 @@ int noalloc_layout(int P, int X, int batch, int dtype, const fw_wigner_desc* d, 
     return fail(FW_EINVAL, "fw_wigner_propagate_noalloc: P and X must be even and in [4, 4096]");
   if (batch < 1 || batch > 65535) return fail(FW_EINVAL, "fw_wigner_propagate_noalloc: batch must be in [1, 65535]");
   L->small = small_shapes(dtype, P, X, batch);
-  L->np = col_parts(dtype, P, X, L->small);
+  L->np = col_parts(dtype, P, X, L->small, batch);
   if (L->np <= 0) return fail(FW_EINVAL, "fw_wigner_propagate_noalloc: unsupported X for the column pass tile");
   const size_t rs = dtype == FW_F64 ? sizeof(double) : sizeof(float);
   L->rvX = row_rv(dtype, X, L->small);
@@ -522,7 +522,9 @@ int noalloc_layout(int P, int X, int batch, int dtype, const fw_wigner_desc* d, 
   L->twP = off;  off += align256(2 * rs * (size_t)P);
   L->twX = off;  off += align256(2 * rs * (size_t)X);
   L->twsX = off; off += align256(2 * rs * (size_t)(L->nsX > 0 ? L->nsX : 1));
-  L->ring = off; off += align256(sizeof(double) * 2 * (size_t)batch * L->np * MMAX);
+  // (the ring is sized for one record per column pair where the generic pass runs)
+  const int recs = col_generic(dtype, P, X) ? X / 2 : L->np;
+  L->ring = off; off += align256(sizeof(double) * 2 * (size_t)batch * recs * MMAX);
   L->tot = off;  off += align256(sizeof(double) * (size_t)batch * MMAX);
   L->wph = off;  off += align256((size_t)4 * P * 2 * rs * (size_t)L->wph_nb);
   L->need = off;

@@ -44,7 +44,9 @@ cudaError_t launch_row_persist(const PassArgs& a, cudaStream_t st);
 cudaError_t launch_col_persist(const PassArgs& a, cudaStream_t st, int* nparts);
 cudaError_t launch_totals(const double* part, int nparts, int M, int batch, double* tot, double* hist,
                           cudaStream_t st);
-int col_parts(int dtype, int P, int X, int small);
+int col_parts(int dtype, int P, int X, int small, int batch);
+int gen_col_parts(int dtype, int P, int X, int batch);
+bool gen_fuses(int dtype, int P);
 int row_rv(int dtype, int N, int small);
 int small_shapes(int dtype, int P, int X, int batch);
 // Wigner plans: any even size in [4, 4096]; the register-resident passes take
@@ -55,6 +57,8 @@ bool col_generic(int dtype, int P, int X);
 inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 cudaError_t launch_generic_row(const PassArgs& a, int dtype, cudaStream_t st);
 cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, int* nparts);
+cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
+                                   long long out_bs, int dtype, cudaStream_t st);
 
 void set_error(const std::string& msg);
 void count_launch(long long n);

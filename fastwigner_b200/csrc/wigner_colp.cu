@@ -414,7 +414,7 @@ bool colp_eligible(const PassArgs& a, int dtype) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   using S = ColpShape<1024>;
-  if (a.X % (2 * S::CP) != 0 || col_parts(dtype, a.P, a.X, 0) != a.X / (2 * S::CP)) return false;
+  if (a.X % (2 * S::CP) != 0 || col_parts(dtype, a.P, a.X, 0, a.batch) != a.X / (2 * S::CP)) return false;
   return (long long)a.batch * (a.X / (2 * S::CP)) >= 2LL * S::MINB * sms && encoder() != nullptr;
 }
 

@@ -179,7 +179,7 @@ static cudaError_t launch_col_n(const PassArgs& a, cudaStream_t st, int* nparts)
 
 // Column passes of sizes the register-resident kernels do not take (P not a
 // power of two in [128, 4096], or X not a multiple of their column tile) run
-// the generic pass, one column pair per CTA.
+// the generic pass.
 static int col_cp(int dtype, int P, int small) {
   int cp = 0;
 #define CPV(R, N) if (P == N) cp = small ? ColCfgSmall<R, N>::CP : ColCfg<R, N>::CP;
@@ -195,11 +195,11 @@ bool col_generic(int dtype, int P, int X) {
   return cp == 0 || X % (2 * cp) != 0 || X % (2 * cps) != 0;
 }
 
-// Partial-sum records per instance of a plan's column passes: X / (2 CP), or
-// X / 2 for the generic pass.
-int col_parts(int dtype, int P, int X, int small) {
+// Partial-sum records per instance of a plan's column passes: X / (2 CP), with
+// the generic pass's CP depending on the batch.
+int col_parts(int dtype, int P, int X, int small, int batch) {
   if (X < 2 || X % 2 != 0) return -1;
-  if (col_generic(dtype, P, X)) return X / 2;
+  if (col_generic(dtype, P, X)) return gen_col_parts(dtype, P, X, batch);
   int cp = 0;
 #define CPV(R, N) if (P == N) cp = small ? ColCfgSmall<R, N>::CP : ColCfg<R, N>::CP;
   if (dtype == FW_F32) { CPV(float, 128) CPV(float, 256) CPV(float, 512) CPV(float, 1024) CPV(float, 2048) CPV(float, 4096) }
@@ -226,7 +226,7 @@ int small_shapes(int dtype, int P, int X, int batch) {
   if (col_generic(dtype, P, X) || !size_pow2_supported(X)) return 0;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int np = col_parts(dtype, P, X, 0);
+  const int np = col_parts(dtype, P, X, 0, batch);
   return np > 0 && (long long)batch * np < sms ? 1 : 0;
 }
 
@@ -315,6 +315,7 @@ __global__ void __launch_bounds__(256) pweight_dft_kernel(const double* wp, long
 
 cudaError_t launch_pweight_dft(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out, long long out_bs,
                                int dtype, cudaStream_t st) {
+  if (!is_pow2(P)) return launch_generic_pweight(wp, wp_bs, Mp, P, nb, out, out_bs, dtype, st);
   const size_t smem = 2 * sizeof(double2) * (size_t)P;
   dim3 grid(Mp, nb);
   cudaError_t e;
