@@ -29,6 +29,7 @@ SOURCES = [
     "expr.cu",
     "fno.cu",
     "fno_umma.cu",
+    "fno_layer.cu",
     "batch.cu",
 ]
 

@@ -47,6 +47,7 @@
 #include <stdint.h>
 #include <string>
 #include "fno_act.cuh"
+#include "fno_umma.cuh"
 #include "fw_internal.h"
 #include "tma.cuh"
 
@@ -78,7 +79,6 @@ struct UmmaArgs {
 
 namespace umma {  // named (external linkage): host helpers take lambdas over these types
 
-constexpr int UM = 128;  // tile rows (tensor-core M)
 constexpr int UK = 32;   // K per shared-memory chunk (four MMAs of K = 8)
 constexpr long long kUmmaMaxPolls = 1LL << 20;
 
@@ -97,51 +97,6 @@ __device__ __forceinline__ uint64_t smem_desc(const void* p, uint32_t lbo_bytes)
   const uint64_t l = (lbo_bytes >> 4) & 0x3FFFu;
   const uint64_t s = (128u >> 4) & 0x3FFFu;
   return a | (l << 16) | (s << 32) | (1ull << 46);
-}
-
-// instruction descriptor of kind::tf32: F32 accumulator, TF32 A and B, both
-// K-major, N = bn, M = 128
-__host__ __device__ constexpr uint32_t instr_desc(int bn) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(UM >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
-      "}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-      : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void proxy_fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&r)[16]) {
-  uint32_t u[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(u[i]);
-}
-
-// TF32 part of x (the 19 leading bits; the tensor core reads no more) and the rest
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-  hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-  lo = x - hi;
 }
 
 // The (row, k-group) that thread (warp, lane) holds as its i-th float4 of a
@@ -613,6 +568,24 @@ int fno_status_read(int* out, int clear) {
     e = cudaMemcpyToSymbol(g_fno_status, &z, sizeof(int));
   }
   return e == cudaSuccess ? FW_OK : cuda_fail(e, "fw_fno_status");
+}
+
+// device address of the status word, looked up once per device
+int fno_status_ptr(int** out) {
+  static int* ptr[kMaxDevices] = {};
+  static PerDeviceOnce once;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = once.run([&] {
+      void* p = nullptr;
+      cudaError_t r = cudaGetSymbolAddress(&p, g_fno_status);
+      if (r == cudaSuccess) ptr[dev] = static_cast<int*>(p);
+      return r;
+    });
+  if (e != cudaSuccess) return cuda_fail(e, "FNO status word");
+  *out = ptr[dev];
+  return FW_OK;
 }
 
 }  // namespace fw

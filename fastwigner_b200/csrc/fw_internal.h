@@ -38,6 +38,7 @@ cudaError_t launch_finalize(const PassArgs& a, int dtype, cudaStream_t st);
 cudaError_t launch_pweight_dft(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out, long long out_bs,
                                int dtype, cudaStream_t st);
 int fno_status_read(int* out, int clear);
+int fno_status_ptr(int** out);
 bool colp_eligible(const PassArgs& a, int dtype);
 bool rowp_eligible(const PassArgs& a, int dtype);
 cudaError_t launch_row_persist(const PassArgs& a, cudaStream_t st);

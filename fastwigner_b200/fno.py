@@ -72,6 +72,29 @@ class _Ops:
         check(self.lib.fw_fno_project(hidden, C, L, _p(V), C * L, batch, _p(Q1), _p(c1), _p(Q2), _p(c2), _p(out), L,
                                       stream_handle()), "fw_fno_project")
 
+    def layer(self, mode, B, G0, G1, W, bias, act=0, vin=None, gx=None, AA=None, CS=None, NP=0, par=None, xs=None,
+              ps=None, Q1=None, c1=None, Q2=None, c2=None, vout=None, fx=None, out=None):
+        opt = lambda t: _p(t) if t is not None else None
+        check(self.lib.fw_fno_layer(mode, B, G0, G1, opt(vin), opt(gx), opt(AA), opt(CS), _p(W), _p(bias), int(act),
+                                    NP, opt(par), opt(xs), opt(ps), opt(Q1), opt(c1), opt(Q2), opt(c2), opt(vout),
+                                    opt(fx), opt(out), stream_handle()), "fw_fno_layer")
+
+    def thermal(self, out, wc, xs, ps, x_e, dxdp):
+        """Thermal states from network outputs (in place), see fw_fno_thermal."""
+        B, G0, G1 = out.shape
+        dp = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        wc = torch.tensor(np.ascontiguousarray(wc, dtype=np.float64), device=out.device)
+        work = torch.empty(64 * B, dtype=torch.float64, device=out.device)
+        check(self.lib.fw_fno_thermal(B, G0, G1, dp(wc), dp(xs), dp(ps), float(x_e), float(dxdp), _p(out), dp(work),
+                                      stream_handle()), "fw_fno_thermal")
+        return out
+
+    def pdft(self, B, G0, G1, fx, Dpv, F2):
+        check(self.lib.fw_fno_pdft(B, G0, G1, _p(fx), _p(Dpv), _p(F2), stream_handle()), "fw_fno_pdft")
+
+    def pidft(self, B, G0, O2, Dpiv, gx):
+        check(self.lib.fw_fno_pidft(B, G0, _p(O2), _p(Dpiv), _p(gx), stream_handle()), "fw_fno_pidft")
+
     def mix(self, mode, B, Ci, Co, K, X, Y, out):
         check(self.lib.fw_fno_mix(mode, B, Ci, Co, K, _p(X), _p(Y), _p(out), stream_handle()), "fw_fno_mix")
 
@@ -200,9 +223,11 @@ class FNO2d:
                           dtype=torch.float32, device=dev).contiguous()
         xs_t = torch.tensor(np.asarray(xs), dtype=torch.float32, device=dev)
         ps_t = torch.tensor(np.asarray(ps), dtype=torch.float32, device=dev)
+        P = self.params
+        if not cache and self._fused_layers(G0, G1):
+            return self._forward_fused(B, G0, G1, pr, xs_t, ps_t)
         feats = torch.empty((B, NP + 2, G0, G1), dtype=torch.float32, device=dev)
         o.features(B, NP, G0, G1, pr, xs_t, ps_t, feats)
-        P = self.params
         v = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
         o.gemm_ex(0, 0, C, L, NP + 2, P["W0"], NP + 2, 0, feats, L, (NP + 2) * L, v, L, C * L, B, bias=P["b0"])
         c = {"B": B, "G0": G0, "G1": G1, "feats": feats, "v": [], "F2": [], "pre": []}
@@ -246,6 +271,34 @@ class FNO2d:
         if cache:
             self._cache = c
         return out.view(B, G0, G1)
+
+    def _fused_layers(self, G0, G1):
+        """Whether the fused layer kernels take this network and grid (fw_fno_layer):
+        the surrogate's own width, modes and projection on any grid they hold."""
+        return (self.C == 32 and self.mp == self.mx == 16 and self.proj == 128 and self.layers >= 1
+                and self.NP <= 14 and 32 <= G0 <= 1024 and G1 >= 32 and G1 % 4 == 0)
+
+    def _forward_fused(self, B, G0, G1, pr, xs_t, ps_t):
+        """Inference: each layer reads and writes the activations once."""
+        o, P, dev, C, K = self.ops, self.params, self.device, self.C, self.K
+        CS, Dpv, Dpiv, AA = self._grid(G0, G1)
+        v = torch.empty((B, G0, G1, C), dtype=torch.float32, device=dev)
+        fx = torch.empty(((G1 + 127) // 128, B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        gx = torch.empty((B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        F2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)
+        O2 = torch.empty_like(F2)
+        out = torch.empty((B, G0, G1), dtype=torch.float32, device=dev)
+        o.layer(0, B, G0, G1, P["W0"], P["b0"], CS=CS, NP=self.NP, par=pr, xs=xs_t, ps=ps_t, vout=v, fx=fx)
+        for l in range(self.layers):
+            o.pdft(B, G0, G1, fx, Dpv, F2)
+            o.mix(0, B, C, C, K, F2, P[f"R{l}"], O2)
+            o.pidft(B, G0, O2, Dpiv, gx)
+            if l < self.layers - 1:
+                o.layer(1, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], act=1, vin=v, gx=gx, AA=AA, CS=CS, vout=v, fx=fx)
+            else:
+                o.layer(2, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], vin=v, gx=gx, AA=AA, Q1=P["Q1"], c1=P["c1"],
+                        Q2=P["Q2"], c2=P["c2"], out=out)
+        return out
 
     # -- backward -----------------------------------------------------------------
     def backward(self, dout):
@@ -496,6 +549,12 @@ class BlochSurrogate:
         B = torch.exp(-c[:, None, None] * (Hh - Hh.amin(dim=(1, 2), keepdim=True)))
         return (B / B.sum(dim=(1, 2), keepdim=True)).float()
 
+    def _grid_device(self):
+        """The full grid's x and p on the device (FP64)."""
+        if getattr(self, "_xp_dev", None) is None:
+            self._xp_dev = tuple(t.to(self.net.device, torch.float64).contiguous() for t in self._xp_full)
+        return self._xp_dev
+
     def train(self, P, S, epochs=20, batch=16, lr=2e-3, rng=None, log=None, group=None):
         """P: (N, 3) raw (D, a, beta); S: (N, g, g) states (normalised to unit sum).
 
@@ -544,9 +603,11 @@ class BlochSurrogate:
                                            np.full(len(Ds[c0:c0 + chunk]), beta)], axis=1))
             out = self.net.forward(X, self.xs, self.ps, cache=False)
             if self.residual:
-                n = len(Ds[c0:c0 + chunk])
-                B = self.baseline(np.stack([Ds[c0:c0 + chunk], As[c0:c0 + chunk], np.full(n, beta)], axis=1))
-                out = B + B.amax(dim=(1, 2), keepdim=True) * out
+                # baseline + its peak x network, normalised (the kernel evaluates baseline())
+                w = As[c0:c0 + chunk] * np.sqrt(2.0 * Ds[c0:c0 + chunk])
+                wc = np.stack([w, (2.0 / w) * np.tanh(0.5 * beta * w)], axis=1)
+                outs.append(self.net.ops.thermal(out, wc, *self._grid_device(), self.s.x_e, self.s.dX * self.s.dP))
+                continue
             outs.append(out / (out.double().sum(dim=(1, 2), keepdim=True) * self.s.dX * self.s.dP).float())
         return torch.cat(outs)
 

@@ -1,0 +1,79 @@
+"""The fused layer kernels of the FNO's inference path (fno_layer.cu) against
+plain FP64 torch, stage by stage, at 1e-5 of each result's maximum (the bound
+of the unfused tensor-core products): one and several x tiles, a ragged last
+tile, fewer and more rows than the GPU has slots; then the whole fused forward
+against the unfused one."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def swizzle(v):
+    """[..., x, 32] <-> the kernels' pixel layout: 4-float piece q of pixel x at q ^ (x & 7)."""
+    x = torch.arange(v.shape[-2], device=v.device)
+    q = torch.arange(8, device=v.device)[None, :] ^ (x[:, None] & 7)
+    idx = (4 * q[:, :, None] + torch.arange(4, device=v.device)).reshape(v.shape[-2], 32)
+    return torch.gather(v, -1, idx.expand(v.shape))
+
+
+def close(a, b, tol=1e-5):
+    assert (a.double() - b).abs().max() <= tol * b.abs().max(), float((a.double() - b).abs().max() / b.abs().max())
+
+
+@pytest.mark.parametrize("B,G0,G1", [(1, 32, 128), (2, 48, 192), (3, 64, 36), (2, 256, 512), (1, 1024, 132)])
+def test_layer_stages(B, G0, G1):
+    from fastwigner_b200.fno import FNO2d
+
+    net = FNO2d(seed=3)
+    o, P = net.ops, net.params
+    CS, Dpv, Dpiv, AA = net._grid(G0, G1)
+    d = lambda t: t.double()  # noqa: E731
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    par, xs, ps = rnd(B, 3), rnd(G1), rnd(G0)
+    v = torch.full((B, G0, G1, 32), float("nan"), device="cuda")
+    fx = torch.full(((G1 + 127) // 128, B * G0, 32, 32), float("nan"), device="cuda")
+    o.layer(0, B, G0, G1, P["W0"], P["b0"], CS=CS, NP=3, par=par, xs=xs, ps=ps, vout=v, fx=fx)
+    feats = torch.cat([par[:, None, None, :].expand(B, G0, G1, 3), xs[None, None, :, None].expand(B, G0, G1, 1),
+                       ps[None, :, None, None].expand(B, G0, G1, 1)], dim=3)
+    v0 = d(feats) @ d(P["W0"]).T + d(P["b0"])
+    close(swizzle(v), v0)
+    close(fx.sum(0).view(B, G0, 32, 32), torch.einsum("bgxc,xk->bgck", v0, d(CS)))
+    # p-transform, its inverse
+    F2 = torch.empty((B, 32, 2, 512), device="cuda")
+    o.pdft(B, G0, G1, fx, Dpv, F2)
+    Fr = fx.double().sum(0).view(B, G0, 32, 2, 16).permute(0, 2, 1, 3, 4).reshape(B, 32, 2 * G0, 16)
+    close(F2, (d(Dpv) @ Fr).reshape(B, 32, 2, 512))
+    gx = torch.empty((B * G0, 32, 32), device="cuda")
+    o.pidft(B, G0, F2, Dpiv, gx)
+    Gr = (d(Dpiv) @ d(F2).reshape(B, 32, 64, 16)).reshape(B, 32, G0, 2, 16).permute(0, 2, 1, 3, 4).reshape(B, G0, 32, 32)
+    close(swizzle(gx).view(B, G0, 32, 32), Gr)
+    # a layer (in place) and the last layer with the projection
+    vin = rnd(B, G0, G1, 32)
+    pre = torch.einsum("bgck,kx->bgxc", Gr, d(AA)) + d(vin) @ d(P["W1"]).T + d(P["b1"])
+    v = swizzle(vin).contiguous()
+    out = torch.full((B, G0, G1), float("nan"), device="cuda")
+    o.layer(2, B, G0, G1, P["W1"], P["b1"], vin=v, gx=gx, AA=AA, Q1=P["Q1"], c1=P["c1"], Q2=P["Q2"], c2=P["c2"], out=out)
+    gelu = torch.nn.functional.gelu
+    close(out, gelu(pre @ d(P["Q1"]).T + d(P["c1"])) @ d(P["Q2"])[0] + d(P["c2"]))
+    o.layer(1, B, G0, G1, P["W1"], P["b1"], act=1, vin=v, gx=gx, AA=AA, CS=CS, vout=v, fx=fx)
+    close(swizzle(v), gelu(pre))
+    close(fx.sum(0).view(B, G0, 32, 32), torch.einsum("bgxc,xk->bgck", gelu(pre), d(CS)))
+    st = ctypes.c_int(7)
+    assert o.lib.fw_fno_status(ctypes.byref(st), 0) == 0 and st.value == 0
+
+
+@pytest.mark.parametrize("G0,G1", [(64, 64), (192, 160), (512, 384)])
+def test_fused_forward_matches_unfused(G0, G1):
+    from fastwigner_b200.fno import FNO2d
+
+    net = FNO2d(seed=1)
+    X = np.random.default_rng(0).uniform(0, 1, (3, 3))
+    xs, ps = np.linspace(-1, 1, G1, endpoint=False), np.linspace(-1, 1, G0, endpoint=False)
+    assert net._fused_layers(G0, G1)
+    a, b = net.forward(X, xs, ps, cache=False), net.forward(X, xs, ps, cache=True)
+    assert (a - b).abs().max() <= 2e-5 * b.abs().max()
