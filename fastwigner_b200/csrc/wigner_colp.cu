@@ -88,10 +88,7 @@ template <int N, int T, int CP, bool PSUM_ALIAS> struct ColpLayout {
 // result).  OBS: the observable sums are taken (a compile-time switch, like
 // the table kind: 0.3127 -> 0.3045 ms per 64 x 1024^2 launch).  v holds
 // the spectrum of the unscaled tile: the input scale sc multiplies the
-// closing factor and the observable sums instead of every element.  The
-// table row min(k, N-k), its Hermitian fold and the mirrored exchange slot of
-// N-k are resolved per m at compile time (k = j + m T, j < T), with the
-// mirror slots one per-thread base minus an immediate.
+// closing factor and the observable sums instead of every element.
 template <int N, int T, int RV, int CP, bool FUSED, bool OBS, typename EX>
 __device__ __forceinline__ void fused_mid_staged(const PassArgs& a, int b, float2 (&v)[RV], const int j, EX& ex,
                                                  int c, const float* Ts, float2* psum, MidSums<float>& o,
@@ -101,72 +98,50 @@ __device__ __forceinline__ void fused_mid_staged(const PassArgs& a, int b, float
                 "folded mirror addressing needs T a multiple of RV and a layout padded per RV");
   const C* G = reinterpret_cast<const C*>(a.wph) + (size_t)b * a.wph_bs;
   constexpr bool obs = OBS;
+  constexpr int H = RV / 2;
   const float hs = (float)(0.5 / (double)N * sc);
-  C u[RV];
-  ex_write_natural<T, RV>(ex, j, v);
-  ex.sync();
+  C u[H];
   o.s2 = 0;
   o.ca = 0;
   o.cb = 0;
 #pragma unroll
   for (int q = 0; q < MAXO; ++q) o.sq[q] = 0;
-  const int mbase = ex.map(N - j);  // slot of N - j (virtual for j = 0); N - k is mbase - delta(m T)
-#pragma unroll
-  for (int m = 0; m < RV; ++m) {
-    // k = j + m T: below N/2 for m < RV/2, else the table holds row N - k (conjugated, except at k = N/2)
-    constexpr int H = RV / 2;
-    const int kk = m < H ? j + m * T : N - j - m * T;
-    C ea, eb;
-    {
-      const float4 e = *reinterpret_cast<const float4*>(Ts + (size_t)kk * (4 * CP) + 4 * c);
-      ea = mk<C>(e.x, e.y);
-      eb = mk<C>(e.z, e.w);
-      if (m == 0 || m == H) {  // k = 0 or k = N/2 when j = 0: real entries
-        if (j == 0) {
-          ea.y = 0.f;
-          eb.y = 0.f;
-        } else if (m == H) {
-          ea.y = -ea.y;
-          eb.y = -eb.y;
-        }
-      } else if (m > H) {
-        ea.y = -ea.y;
-        eb.y = -eb.y;
-      }
-    }
-    const int ms = m == 0 ? (j == 0 ? ex.map(0) : mbase) : mbase - EX::delta(m * T);
-    const C zc = cconj(ex.read_at(ms));
-    const C A = cmul(cadd(v[m], zc), ea);   // 2/sc x spectrum of column a at the mid-point
-    const C Bi = cmul(csub(v[m], zc), eb);  // 2i/sc x spectrum of column b at the mid-point
+  const float* tj = Ts + (size_t)j * (4 * CP) + 4 * c;
+  pair_mid<N, T, RV>(v, j, ex, [&](int m, int k, C& A, C& Bi) {
+    const float4 e = *reinterpret_cast<const float4*>(m < H ? tj + m * T * (4 * CP) : Ts + (size_t)(N / 2) * (4 * CP) + 4 * c);
+    C ea = mk<C>(e.x, e.y), eb = mk<C>(e.z, e.w);
+    if (k == 0 || m == H) ea.y = eb.y = 0.f;
+    A = cmul(A, ea);    // 2/sc x spectrum of column a at the mid-point
+    Bi = cmul(Bi, eb);  // 2i/sc x spectrum of column b at the mid-point
     if (obs) {
-      o.s2 += (double)(A.x * A.x + A.y * A.y + Bi.x * Bi.x + Bi.y * Bi.y);
+      const double s2 = (double)(A.x * A.x + A.y * A.y + Bi.x * Bi.x + Bi.y * Bi.y);
+      o.s2 += (k == 0 || m == H) ? s2 : 2.0 * s2;
       if (m == 0 && j == 0) {
         o.ca = A.x;
         o.cb = Bi.y;
       }
-      u[m] = mk<C>(A.x + Bi.y, A.y - Bi.x);  // 2/sc x (spectrum a + spectrum b)
+      const C w = mk<C>(A.x + Bi.y, A.y - Bi.x);  // 2/sc x (spectrum a + spectrum b)
+      if (m < H) {
+        u[m < H ? m : 0] = w;
+      } else if (a.Mp > 0) {
+        const C t = dc_lanes_sum<CP>(w);
+        if (c == 0) psum[N / 2] = t;
+      }
     }
     // fused: close step k and open step k+1 with the same factor; a single
     // half-step (the opening one of a call, or its closing one) repacks A, Bi
-    v[m] = FUSED ? cscale(cadd(cmul(A, ea), cmul(Bi, eb)), hs) : cscale(cadd(A, Bi), hs);
-  }
-  // per-bin sums over the tile's CP column pairs; lane c ends with bins
-  // m = c * RV/CP + i
-  if (obs && a.Mp > 0) halving_sum<CP, RV>(u, c);
-  ex.sync();  // the table tile and the exchange buffer are no longer read
+    A = FUSED ? cscale(cmul(A, ea), hs) : cscale(A, hs);
+    Bi = FUSED ? cscale(cmul(Bi, eb), hs) : cscale(Bi, hs);
+  });
   if (obs && a.Mp > 0) {
+    // per-bin sums over the tile's CP column pairs; lane c ends with bins
+    // m = c * H/CP + i
+    halving_sum<CP, H>(u, c);
 #pragma unroll
-    for (int i = 0; i < RV / CP; ++i) psum[j + (c * (RV / CP) + i) * T] = u[i];
-    ex.sync();
-    for (int k = threadIdx.x; k < N; k += blockDim.x) {
-      const C u = psum[k];
-      C g[MAXO];
-      load_bin_weights<float>(G + (size_t)k * MAXO, a.Mp, g);
-#pragma unroll
-      for (int q = 0; q < MAXO; ++q)
-        if (q < a.Mp) o.sq[q] += (double)u.x * (double)g[q].x + (double)u.y * (double)g[q].y;
-    }
+    for (int i = 0; i < H / CP; ++i) psum[j + (c * (H / CP) + i) * T] = u[i];
   }
+  ex.sync();  // the table tile and the exchange buffer are no longer read
+  if (obs && a.Mp > 0) bin_weights<float, N>(G, a.Mp, psum, threadIdx.x, CP * T, o);
   if (obs) {  // the sums of the unscaled spectrum, scaled once
     o.s2 *= sc * sc;
     o.ca *= sc;

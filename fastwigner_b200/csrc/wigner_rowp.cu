@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 1) row_persist_kernel(PassArgs
   bool w_pending = true, t_pending = kRowStageTable, failed = false;
   GroupExC<float, T> ex{exz};
   const int j = lane;
-  const float f = (float)(a.out_scale / (double)N);
+  const float fh = (float)(0.5 * a.out_scale / (double)N);
 
   for (int it = first; it < last; ++it) {
     const int rp = ipair(it), b = iinst(it);
@@ -120,46 +120,18 @@ __global__ void __launch_bounds__(32 * kRowWarps, 1) row_persist_kernel(PassArgs
       ph_t ^= 1u;
       t_pending = false;
     }
-    ex_write_natural<T, RV>(ex, j, v);
-    ex.sync();
     const C* tab = kRowStageTable
                        ? Ts
                        : reinterpret_cast<const C*>(a.tab1) + (size_t)b * a.tab_bs + (size_t)(2 * rp) * HS;
-    // bin k = j + m T: table row k below N/2 (m < RV/2), row N - k conjugated
-    // above it, at m = RV/2 row N/2 - j (N/2 itself, real, for j = 0); the
-    // mirrored exchange slot of N - k is one per-thread base minus an
-    // immediate, except k = 0 (slot 0).  Resolved per m at compile time: the
-    // row pass from 0.1648 to 0.1584 ms per 64 x 1024^2 launch.
-    const C* tlo = tab + j;
-    const C* thi = tab + (N - j);
     auto ld = [&](const C* p) { return kRowStageTable ? *p : __ldg(p); };
-    const int mbase = GroupExC<float, T>::map(N - j);
-#pragma unroll
-    for (int m = 0; m < RV; ++m) {
-      constexpr int H = RV / 2;
-      C ea, eb;
-      if (m < H) {
-        ea = ld(tlo + m * T);
-        eb = ld(tlo + HS + m * T);
-        if (m == 0 && j == 0) {
-          ea.y = 0.f;
-          eb.y = 0.f;
-        }
-      } else {
-        ea = ld(thi - m * T);
-        eb = ld(thi + HS - m * T);
-        if (m == H && j == 0) {
-          ea.y = 0.f;
-          eb.y = 0.f;
-        } else {
-          ea.y = -ea.y;
-          eb.y = -eb.y;
-        }
-      }
-      const int ms = m == 0 ? (j == 0 ? 0 : mbase) : mbase - GroupExC<float, T>::delta(m * T);
-      const C znk = ex.read_at(ms);
-      v[m] = two_real_mul(v[m], znk, ea, eb, f);
-    }
+    const C* tj = tab + j;
+    pair_mid<N, T, RV>(v, j, ex, [&](int m, int k, C& X, C& Y) {
+      const C* t = m < RV / 2 ? tj + m * T : tab + N / 2;
+      C ea = ld(t), eb = ld(t + HS);
+      if (k == 0 || m == RV / 2) ea.y = eb.y = 0.f;
+      X = cscale(cmul(X, ea), fh);
+      Y = cscale(cmul(Y, eb), fh);
+    });
     ex.sync();  // every lane is done with Ts and the exchange buffer
     if (kRowStageTable && it + 1 < last && tkey(it + 1) != tkey(it)) {
       if (lane == 0) issue_t(it + 1);

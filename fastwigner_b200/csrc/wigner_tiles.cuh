@@ -7,23 +7,21 @@
 namespace fw {
 
 // ---------------------------------------------------------------------------
-// Factors of the two packed sequences at full-spectrum index k: table entries
-// kk = min(k, N-k) (taba/tabb, tab_stride apart), times g[kk] when g is given,
-// Hermitian-extended.
+// Factors of the two packed sequences at bin k <= N/2: table entries k
+// (taba/tabb, tab_stride apart), times g[k] when g is given; real at k = 0 and
+// N/2 (a complex-to-real transform drops those imaginary parts).
 template <typename Rl, int N>
 __device__ __forceinline__ void factor_pair(const void* taba, const void* tabb, size_t tab_stride, int tab_real,
                                             const void* g, int k, cplx_t<Rl>& ea, cplx_t<Rl>& eb) {
   using C = cplx_t<Rl>;
-  const int kk = (k <= N / 2) ? k : N - k;
-  ea = tab_load<Rl>(taba, tab_real, (size_t)kk * tab_stride);
-  eb = tab_load<Rl>(tabb, tab_real, (size_t)kk * tab_stride);
+  ea = tab_load<Rl>(taba, tab_real, (size_t)k * tab_stride);
+  eb = tab_load<Rl>(tabb, tab_real, (size_t)k * tab_stride);
   if (g != nullptr) {
-    const C gk = __ldg(reinterpret_cast<const C*>(g) + kk);
+    const C gk = __ldg(reinterpret_cast<const C*>(g) + k);
     ea = cmul(ea, gk);
     eb = cmul(eb, gk);
   }
-  ea = herm(ea, k, N);
-  eb = herm(eb, k, N);
+  if (k == 0 || k == N / 2) ea.y = eb.y = 0;
 }
 
 // factor_pair for a column pair whose two entries are adjacent in a table
@@ -33,34 +31,32 @@ template <typename Rl, int N>
 __device__ __forceinline__ void factor_pair_vec(const void* taba, size_t tab_stride, int tab_real, const void* g,
                                                 int k, cplx_t<Rl>& ea, cplx_t<Rl>& eb) {
   using C = cplx_t<Rl>;
-  const int kk = (k <= N / 2) ? k : N - k;
   if constexpr (sizeof(Rl) == 4) {
     if (tab_real) {
-      const float2 e = __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(taba) + kk * tab_stride));
+      const float2 e = __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(taba) + k * tab_stride));
       ea = mk<C>(e.x, 0.f);
       eb = mk<C>(e.y, 0.f);
     } else {
-      const float4 e = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(taba) + kk * tab_stride));
+      const float4 e = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(taba) + k * tab_stride));
       ea = mk<C>(e.x, e.y);
       eb = mk<C>(e.z, e.w);
     }
   } else {
     if (tab_real) {
-      const double2 e = __ldg(reinterpret_cast<const double2*>(reinterpret_cast<const double*>(taba) + kk * tab_stride));
+      const double2 e = __ldg(reinterpret_cast<const double2*>(reinterpret_cast<const double*>(taba) + k * tab_stride));
       ea = mk<C>(e.x, 0.0);
       eb = mk<C>(e.y, 0.0);
     } else {
-      ea = __ldg(reinterpret_cast<const C*>(taba) + kk * tab_stride);
-      eb = __ldg(reinterpret_cast<const C*>(taba) + kk * tab_stride + 1);
+      ea = __ldg(reinterpret_cast<const C*>(taba) + k * tab_stride);
+      eb = __ldg(reinterpret_cast<const C*>(taba) + k * tab_stride + 1);
     }
   }
   if (g != nullptr) {
-    const C gk = __ldg(reinterpret_cast<const C*>(g) + kk);
+    const C gk = __ldg(reinterpret_cast<const C*>(g) + k);
     ea = cmul(ea, gk);
     eb = cmul(eb, gk);
   }
-  ea = herm(ea, k, N);
-  eb = herm(eb, k, N);
+  if (k == 0 || k == N / 2) ea.y = eb.y = 0;
 }
 
 // The first n (<= MAXO) p-weight spectra at one bin ([k][q] layout, 4 entries,
@@ -85,37 +81,69 @@ __device__ __forceinline__ void load_bin_weights(const cplx_t<Rl>* gk, int n, cp
   }
 }
 
+// Spectral mid-point of a packed pair a + i b: v holds the natural-order
+// spectrum Z (bins k = j + m T).  mul(m, k, X, Y) turns X = Z_k + conj Z_(N-k) and
+// Y = Z_k - conj Z_(N-k) (2 x the spectrum of a, 2i x that of b) into their
+// products with the factors at bin k; then bin k becomes X + Y and bin N - k
+// conj(X - Y).  The factors of the two bins are conjugates, so the thread that
+// holds the lower bin does both: half the factor loads and products of a
+// multiply bin by bin.  The upper halves travel through the exchange buffer,
+// there to their lower bin's thread and back in the same slot.  On return the
+// upper halves have been read but not every thread need have done so: the
+// caller synchronises before the buffer is written again.
+// (Bin by bin, the headline step's two passes took 0.289 + 0.158 ms.)
+template <int N, int T, int RV, typename EX, typename C, typename Mul>
+__device__ __forceinline__ void pair_mid(C (&v)[RV], const int j, const EX& ex, Mul mul) {
+  constexpr int H = RV / 2;
+  constexpr bool FOLD = EX::kFold && EX::kL == ilog2_c(RV) && T >= RV;
+  // When T is a multiple of the exchange's padding period, the slot of N - k
+  // is one per-thread base minus an immediate for every m.
+  constexpr bool MIRROR = EX::kFold && T % (1 << EX::kL) == 0;
+  const int aj = ex.map(j);
+  const int mbase = MIRROR ? ex.map(N - j) : 0;  // virtual slot of N for j = 0
+#pragma unroll
+  for (int m = H; m < RV; ++m) ex.write_at(FOLD ? aj + EX::delta(m * T) : ex.map(j + m * T), v[m]);
+  ex.sync();
+#pragma unroll
+  for (int m = 0; m < H; ++m) {
+    const int k = j + m * T;
+    const bool self = m == 0 && j == 0;  // bin 0 pairs with itself
+    const int sn = self ? ex.map(N / 2) : MIRROR ? mbase - EX::delta(m * T) : ex.map(N - k);
+    C zc = ex.read_at(sn);
+    if (self) zc = v[0];
+    zc = cconj(zc);
+    C X = cadd(v[m], zc), Y = csub(v[m], zc);
+    mul(m, k, X, Y);
+    v[m] = cadd(X, Y);
+    if (!self) ex.write_at(sn, cconj(csub(X, Y)));
+  }
+  if (j == 0) {  // so does bin N/2
+    const C zc = cconj(v[H]);
+    C X = cadd(v[H], zc), Y = csub(v[H], zc);
+    mul(H, N / 2, X, Y);
+    ex.write_at(ex.map(N / 2), cadd(X, Y));
+  }
+  ex.sync();
+#pragma unroll
+  for (int m = H; m < RV; ++m) v[m] = ex.read_at(FOLD ? aj + EX::delta(m * T) : ex.map(j + m * T));
+}
+
 // Spectral multiply between a forward and an inverse transform (shared by the
-// row and column passes).  v holds the natural-order spectrum Z of a + i b.
-// taba/tabb point at the half-spectrum factors of the two packed sequences;
-// tab_stride is the distance between consecutive half-spectrum entries.
+// row and column passes).  taba/tabb point at the half-spectrum factors of the
+// two packed sequences; tab_stride is the distance between consecutive
+// half-spectrum entries.
 template <typename Rl, int N, int T, int RV, typename EX>
 __device__ __forceinline__ void spectral_mul(cplx_t<Rl> (&v)[RV], const int j, EX& ex, const void* taba,
                                              const void* tabb, size_t tab_stride, int tab_real, const void* g,
                                              Rl f) {
   using C = cplx_t<Rl>;
-  ex_write_natural<T, RV>(ex, j, v);
-  ex.sync();
-  // When T is a multiple of the exchange's padding period, the slot of N - k
-  // (k = j + m T) is one per-thread base minus an immediate for every m
-  // (slot of 0 for k = 0), as in the persistent passes (Bloch 512^2 FP32,
-  // 16 instances: 0.0553 -> 0.0514 ms per step; the uneven batch 0.634 ->
-  // 0.620 ms).
-  constexpr bool kFoldMirror = EX::kFold && T % (1 << EX::kL) == 0;
-  const int mbase = kFoldMirror ? ex.map(N - j) : 0;  // virtual slot of N for j = 0
-#pragma unroll
-  for (int m = 0; m < RV; ++m) {
-    const int k = j + m * T;
+  const Rl h = f * (Rl)0.5;
+  pair_mid<N, T, RV>(v, j, ex, [&](int, int k, C& X, C& Y) {
     C ea, eb;
     factor_pair<Rl, N>(taba, tabb, tab_stride, tab_real, g, k, ea, eb);
-    C znk;
-    if constexpr (kFoldMirror) {
-      znk = ex.read_at(m == 0 ? (j == 0 ? ex.map(0) : mbase) : mbase - EX::delta(m * T));
-    } else {
-      znk = ex.read((N - k) & (N - 1));
-    }
-    v[m] = two_real_mul(v[m], znk, ea, eb, f);
-  }
+    X = cscale(cmul(X, ea), h);
+    Y = cscale(cmul(Y, eb), h);
+  });
   ex.sync();
 }
 
@@ -215,12 +243,76 @@ __device__ __forceinline__ void col_store(const PassArgs& a, const cplx_t<Rl> (&
 // Per-thread partial sums of a fused column pass, accumulated in FP64 whatever
 // the state precision: sum |2A_k|^2 + |2B_k|^2 over the thread's bins (each
 // bin's four squares summed in the state precision -- positive terms, so
-// that short sum has no cancellation -- then added in FP64), sum
-// Re(2(A_k+B_k) conj(Wh_k)) per p-weight, and (thread j == 0 only) the
-// doubled DC bins of the pair.
+// that short sum has no cancellation -- then added in FP64; bins k and N - k are
+// conjugates and count twice), sum Re(2(A_k+B_k) conj(Wh_k)) per p-weight, and
+// (thread j == 0 only) the doubled DC bins of the pair.
 template <typename Rl> struct MidSums {
   double s2, sq[MAXO], ca, cb;
 };
+
+// Sum over the CP column pairs (adjacent lanes c) of PB values per lane, one
+// bin each: the first log2(PB) shuffle levels scatter the block (a lane keeps
+// half of its values and sends the other half), the rest sum one value; on
+// return kp is the sum of value vi, complete in lanes with c % (CP/PB) == 0.
+// (FP64 256^2, batch 512: 0.5266 -> 0.5070 ms per step against a full butterfly
+// per bin.)
+template <int CP, int PB, typename C>
+__device__ __forceinline__ void bins_sum(const C (&ub)[PB], int c, C& kp, int& vi) {
+  static_assert(PB == 1 || PB == 2 || PB == 4, "1, 2 or 4 bins");
+  kp = ub[0];
+  vi = 0;
+  if constexpr (PB == 4) {
+    const bool up = (c & (CP / 2)) != 0, up2 = (c & (CP / 4)) != 0;
+    C k0 = up ? ub[2] : ub[0], k1 = up ? ub[3] : ub[1];
+    const C s0 = up ? ub[0] : ub[2], s1 = up ? ub[1] : ub[3];
+    k0 = cadd(k0, mk<C>(__shfl_xor_sync(0xffffffffu, s0.x, CP / 2), __shfl_xor_sync(0xffffffffu, s0.y, CP / 2)));
+    k1 = cadd(k1, mk<C>(__shfl_xor_sync(0xffffffffu, s1.x, CP / 2), __shfl_xor_sync(0xffffffffu, s1.y, CP / 2)));
+    kp = up2 ? k1 : k0;
+    const C s = up2 ? k0 : k1;
+    kp = cadd(kp, mk<C>(__shfl_xor_sync(0xffffffffu, s.x, CP / 4), __shfl_xor_sync(0xffffffffu, s.y, CP / 4)));
+    vi = (up ? 2 : 0) + (up2 ? 1 : 0);
+  } else if constexpr (PB == 2) {
+    const bool up = (c & (CP / 2)) != 0;
+    kp = up ? ub[1] : ub[0];
+    const C s = up ? ub[0] : ub[1];
+    kp = cadd(kp, mk<C>(__shfl_xor_sync(0xffffffffu, s.x, CP / 2), __shfl_xor_sync(0xffffffffu, s.y, CP / 2)));
+    vi = up ? 1 : 0;
+  }
+#pragma unroll
+  for (int off = CP / (2 * PB); off > 0; off >>= 1) {
+    kp.x += __shfl_xor_sync(0xffffffffu, kp.x, off);
+    kp.y += __shfl_xor_sync(0xffffffffu, kp.y, off);
+  }
+}
+
+// u summed over the CP lanes of j == 0 (lanes 0 .. CP-1 of warp 0; only they call).
+template <int CP, typename C> __device__ __forceinline__ C dc_lanes_sum(C u) {
+  constexpr unsigned mask = CP >= 32 ? 0xffffffffu : (1u << CP) - 1u;
+#pragma unroll
+  for (int off = CP / 2; off > 0; off >>= 1) {
+    u.x += __shfl_xor_sync(mask, u.x, off);
+    u.y += __shfl_xor_sync(mask, u.y, off);
+  }
+  return u;
+}
+
+// The p-weight sums of a tile from its per-bin sums psum[0 .. N/2], each
+// bin's weight spectra loaded once (thread t of n).
+template <typename Rl, int N>
+__device__ __forceinline__ void bin_weights(const cplx_t<Rl>* G, int Mp, const cplx_t<Rl>* psum, int t, int n,
+                                            MidSums<Rl>& o) {
+  using C = cplx_t<Rl>;
+  for (int k = t; k <= N / 2; k += n) {
+    const C u = psum[k];
+    const double w = (k == 0 || k == N / 2) ? 1.0 : 2.0;
+    const double ux = w * (double)u.x, uy = w * (double)u.y;
+    C g[MAXO];
+    load_bin_weights<Rl>(G + (size_t)k * MAXO, Mp, g);
+#pragma unroll
+    for (int q = 0; q < MAXO; ++q)
+      if (q < Mp) o.sq[q] += ux * (double)g[q].x + uy * (double)g[q].y;
+  }
+}
 
 // Mid-point of a fused column pass (a.fuse_mid): v holds the forward spectrum
 // Z of the column pair a + i b (columns xa, xa+1).  Split Z into the two real
@@ -242,20 +334,15 @@ __device__ __forceinline__ void fused_mid(const PassArgs& a, int b, cplx_t<Rl> (
   const C* G = reinterpret_cast<const C*>(a.wph) + (size_t)b * a.wph_bs;
   const bool obs = a.part_out != nullptr;
   const Rl h = (Rl)(0.5 / (double)N);
-  ex_write_natural<T, RV>(ex, j, v);
-  ex.sync();
   o.s2 = 0;
   o.ca = 0;
   o.cb = 0;
 #pragma unroll
   for (int q = 0; q < MAXO; ++q) o.sq[q] = 0;
-  // bins per block of the paired per-bin reduction (at most CP)
-  constexpr int PB = CP >= 4 ? 4 : (CP >= 2 ? 2 : 1);
-  static_assert(RV % PB == 0, "bin blocks must tile the thread's bins");
+  // bins per block of the per-bin reduction (at most CP)
+  constexpr int H = RV / 2, PB = (CP >= 4 && H % 4 == 0) ? 4 : (CP >= 2 && H % 2 == 0 ? 2 : 1);
   C ub[PB];
-#pragma unroll
-  for (int m = 0; m < RV; ++m) {
-    const int k = j + m * T;
+  pair_mid<N, T, RV>(v, j, ex, [&](int m, int k, C& A, C& Bi) {
     C ea1, eb1, ea2, eb2;
     if (a.tab_vec) {
       factor_pair_vec<Rl, N>(t1, (size_t)X, a.tab_real, a.g1, k, ea1, eb1);
@@ -270,67 +357,37 @@ __device__ __forceinline__ void fused_mid(const PassArgs& a, int b, cplx_t<Rl> (
     } else {
       factor_pair<Rl, N>(t2, t2 + esz, (size_t)X, a.tab_real, a.g2, k, ea2, eb2);
     }
-    const C zc = cconj(ex.read((N - k) & (N - 1)));
-    const C A = cmul(cadd(v[m], zc), ea1);   // 2 x spectrum of column a at the mid-point
-    const C Bi = cmul(csub(v[m], zc), eb1);  // 2i x spectrum of column b at the mid-point
+    A = cmul(A, ea1);    // 2 x spectrum of column a at the mid-point
+    Bi = cmul(Bi, eb1);  // 2i x spectrum of column b at the mid-point
     if (obs) {
-      o.s2 += (double)(A.x * A.x + A.y * A.y + Bi.x * Bi.x + Bi.y * Bi.y);
+      const double s2 = (double)(A.x * A.x + A.y * A.y + Bi.x * Bi.x + Bi.y * Bi.y);
+      o.s2 += (k == 0 || m == H) ? s2 : 2.0 * s2;
       if (m == 0 && j == 0) {  // DC bin: the column sums
         o.ca = A.x;
         o.cb = Bi.y;
       }
       if (a.Mp > 0) {
         // 2 x (spectrum a + spectrum b), summed over the tile's CP column pairs
-        // (lanes c of one row group are adjacent) for a block of PB bins at a
-        // time: the first log2(PB) shuffle levels scatter the block (a lane
-        // keeps half of its values and sends the other half), the rest sum one
-        // value, and one lane per bin stores it (FP64 256^2, batch 512: 0.5266 ->
-        // 0.5070 ms per step against a full butterfly per bin)
-        ub[m % PB] = mk<C>(A.x + Bi.y, A.y - Bi.x);
-        if (m % PB == PB - 1) {
-          C kp = ub[0];
-          int vi = 0;
-          if constexpr (PB == 4) {
-            const bool up = (c & (CP / 2)) != 0, up2 = (c & (CP / 4)) != 0;
-            C k0 = up ? ub[2] : ub[0], k1 = up ? ub[3] : ub[1];
-            const C s0 = up ? ub[0] : ub[2], s1 = up ? ub[1] : ub[3];
-            k0 = cadd(k0, mk<C>(__shfl_xor_sync(0xffffffffu, s0.x, CP / 2), __shfl_xor_sync(0xffffffffu, s0.y, CP / 2)));
-            k1 = cadd(k1, mk<C>(__shfl_xor_sync(0xffffffffu, s1.x, CP / 2), __shfl_xor_sync(0xffffffffu, s1.y, CP / 2)));
-            kp = up2 ? k1 : k0;
-            const C s = up2 ? k0 : k1;
-            kp = cadd(kp, mk<C>(__shfl_xor_sync(0xffffffffu, s.x, CP / 4), __shfl_xor_sync(0xffffffffu, s.y, CP / 4)));
-            vi = (up ? 2 : 0) + (up2 ? 1 : 0);
-          } else if constexpr (PB == 2) {
-            const bool up = (c & (CP / 2)) != 0;
-            kp = up ? ub[1] : ub[0];
-            const C s = up ? ub[0] : ub[1];
-            kp = cadd(kp, mk<C>(__shfl_xor_sync(0xffffffffu, s.x, CP / 2), __shfl_xor_sync(0xffffffffu, s.y, CP / 2)));
-            vi = up ? 1 : 0;
+        const C u = mk<C>(A.x + Bi.y, A.y - Bi.x);
+        if (m < H) {
+          ub[m % PB] = u;
+          if (m % PB == PB - 1) {
+            C kp;
+            int vi;
+            bins_sum<CP, PB>(ub, c, kp, vi);
+            if ((c & (CP / PB - 1)) == 0) psum[j + (m - (PB - 1) + vi) * T] = kp;
           }
-#pragma unroll
-          for (int off = CP / (2 * PB); off > 0; off >>= 1) {
-            kp.x += __shfl_xor_sync(0xffffffffu, kp.x, off);
-            kp.y += __shfl_xor_sync(0xffffffffu, kp.y, off);
-          }
-          if ((c & (CP / PB - 1)) == 0) psum[j + (m - (PB - 1) + vi) * T] = kp;
+        } else {
+          const C s = dc_lanes_sum<CP>(u);
+          if (c == 0) psum[N / 2] = s;
         }
       }
     }
-    v[m] = cscale(cadd(cmul(A, ea2), cmul(Bi, eb2)), h);
-  }
+    A = cscale(cmul(A, ea2), h);
+    Bi = cscale(cmul(Bi, eb2), h);
+  });
+  if (obs && a.Mp > 0) bin_weights<Rl, N>(G, a.Mp, psum, threadIdx.x, blockDim.x, o);
   ex.sync();
-  if (obs && a.Mp > 0) {
-    // the p-weight sums: each bin's tile sum against its weight spectra, the
-    // weights loaded once per bin and CTA
-    for (int k = threadIdx.x; k < N; k += blockDim.x) {
-      const C u = psum[k];
-      C g[MAXO];
-      load_bin_weights<Rl>(G + (size_t)k * MAXO, a.Mp, g);
-#pragma unroll
-      for (int q = 0; q < MAXO; ++q)
-        if (q < a.Mp) o.sq[q] += (double)u.x * (double)g[q].x + (double)u.y * (double)g[q].y;
-    }
-  }
 }
 
 // Reduce MidSums over the CTA (column-interleaved layout: lane c of a row
