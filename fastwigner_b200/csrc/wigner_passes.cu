@@ -84,39 +84,44 @@ __global__ void finalize_kernel(PassArgs a, int vec) {
 }
 
 // ---------------------------------------------------------------------------
-// Launch configuration per FFT length and precision (column passes above
-// N = 1024 FP32 / 512 FP64 use 256-thread CTAs so that a thread may hold 255
-// registers: the 32-value transforms spill badly at 128).
+// Launch configuration per FFT length and precision.  MINB is what sets the
+// registers per thread: two to six CTAs per SM (85 to 128 registers, a few
+// spilled) beat one CTA of threads that hold everything, because these passes wait
+// on loads and exchanges.  Per launch, before and after, us (512 x 128^2, 512 x 256^2,
+// 32 x 512^2, 8 x 1024^2, 4 x 2048^2): FP64 column 88.3 -> 57.3, 267 -> 190.6, 90.0 -> 65.6,
+// 102.4 -> 77.8, 295 -> 243.6; FP64 row 53.3 -> 51.2, 135.2 -> 133.1, 55.3 -> 47.1; FP32 (512 x 128^2,
+// 256 x 256^2, 4 x 2048^2) column 49.1 -> 38.9, 98.3 -> 73.8, 167.9 -> 137.9, row 41.0 -> 37.0,
+// 61.5 -> 55.3, 77.9 -> 62.3.  More CTAs still were slower (FP64 256 at five: 266).
 template <typename Rl, int N> struct RowCfg;
 template <typename Rl, int N> struct ColCfg;
 // float: T threads per transform, RV = N / T values per thread
-template <> struct RowCfg<float, 128> { static constexpr int T = 16, G = 16, MINB = 1; };
-template <> struct RowCfg<float, 256> { static constexpr int T = 32, G = 4, MINB = 2; };
+template <> struct RowCfg<float, 128> { static constexpr int T = 16, G = 16, MINB = 3; };
+template <> struct RowCfg<float, 256> { static constexpr int T = 32, G = 4, MINB = 6; };
 template <> struct RowCfg<float, 512> { static constexpr int T = 32, G = 4, MINB = 2; };
 template <> struct RowCfg<float, 1024> { static constexpr int T = 32, G = 4, MINB = 3; };
-template <> struct RowCfg<float, 2048> { static constexpr int T = 64, G = 4, MINB = 1; };
-template <> struct RowCfg<float, 4096> { static constexpr int T = 128, G = 2, MINB = 1; };
-template <> struct RowCfg<double, 128> { static constexpr int T = 16, G = 16, MINB = 1; };
-template <> struct RowCfg<double, 256> { static constexpr int T = 16, G = 8, MINB = 2; };
-template <> struct RowCfg<double, 512> { static constexpr int T = 32, G = 8, MINB = 1; };
+template <> struct RowCfg<float, 2048> { static constexpr int T = 64, G = 2, MINB = 4; };
+template <> struct RowCfg<float, 4096> { static constexpr int T = 128, G = 2, MINB = 2; };
+template <> struct RowCfg<double, 128> { static constexpr int T = 16, G = 16, MINB = 3; };
+template <> struct RowCfg<double, 256> { static constexpr int T = 16, G = 8, MINB = 4; };
+template <> struct RowCfg<double, 512> { static constexpr int T = 32, G = 8, MINB = 2; };
 template <> struct RowCfg<double, 1024> { static constexpr int T = 64, G = 4, MINB = 1; };
 template <> struct RowCfg<double, 2048> { static constexpr int T = 128, G = 2, MINB = 1; };
 template <> struct RowCfg<double, 4096> { static constexpr int T = 256, G = 1, MINB = 1; };
 
-template <> struct ColCfg<float, 128> { static constexpr int T = 16, CP = 32, MINB = 1; };
-template <> struct ColCfg<float, 256> { static constexpr int T = 32, CP = 16, MINB = 1; };
+template <> struct ColCfg<float, 128> { static constexpr int T = 16, CP = 32, MINB = 2; };
+template <> struct ColCfg<float, 256> { static constexpr int T = 32, CP = 16, MINB = 2; };
 template <> struct ColCfg<float, 512> { static constexpr int T = 32, CP = 16, MINB = 1; };
 // 1024: the column tile of the persistent column pass (wigner_colp.cu), which
 // writes the same partial-sum records
 template <> struct ColCfg<float, 1024> { static constexpr int T = 64, CP = 8, MINB = 1; };
-template <> struct ColCfg<float, 2048> { static constexpr int T = 64, CP = 4, MINB = 1; };
-template <> struct ColCfg<float, 4096> { static constexpr int T = 128, CP = 2, MINB = 1; };
-template <> struct ColCfg<double, 128> { static constexpr int T = 16, CP = 16, MINB = 1; };
-template <> struct ColCfg<double, 256> { static constexpr int T = 16, CP = 8, MINB = 2; };
-template <> struct ColCfg<double, 512> { static constexpr int T = 32, CP = 8, MINB = 1; };
-template <> struct ColCfg<double, 1024> { static constexpr int T = 64, CP = 4, MINB = 1; };
-template <> struct ColCfg<double, 2048> { static constexpr int T = 128, CP = 2, MINB = 1; };
-template <> struct ColCfg<double, 4096> { static constexpr int T = 256, CP = 1, MINB = 1; };
+template <> struct ColCfg<float, 2048> { static constexpr int T = 64, CP = 4, MINB = 2; };
+template <> struct ColCfg<float, 4096> { static constexpr int T = 128, CP = 2, MINB = 2; };
+template <> struct ColCfg<double, 128> { static constexpr int T = 16, CP = 16, MINB = 3; };
+template <> struct ColCfg<double, 256> { static constexpr int T = 16, CP = 8, MINB = 4; };
+template <> struct ColCfg<double, 512> { static constexpr int T = 32, CP = 8, MINB = 2; };
+template <> struct ColCfg<double, 1024> { static constexpr int T = 64, CP = 4, MINB = 2; };
+template <> struct ColCfg<double, 2048> { static constexpr int T = 128, CP = 2, MINB = 2; };
+template <> struct ColCfg<double, 4096> { static constexpr int T = 256, CP = 1, MINB = 2; };
 
 // Shapes for batches whose column pass would leave SMs idle with the shapes
 // above (the one-instance use of the drop-in classes): the same shapes unless
