@@ -13,6 +13,11 @@ namespace fw {
 static thread_local std::string g_err;
 void set_error(const std::string& msg) { g_err = msg; }
 int fail(int code, const std::string& msg) { set_error(msg); return code; }
+int dep_launches(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+}
+
 int cuda_fail(cudaError_t e, const char* where) {
   return fail(FW_ECUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
@@ -230,6 +235,7 @@ extern "C" int fw_wigner_propagate(fw_wigner_plan* plan, const fw_wigner_desc* d
   base.out_scale = 1.0;
   base.small_shape = plan->small;
   base.status = plan->status;
+  base.dep = dep_launches(st);
 
   auto tabV = [&](int k) { return advance(d->tabV, (long long)k * d->tabV_step, tes); };
   auto tabK = [&](int k) { return advance(d->tabK, (long long)k * d->tabK_step, tes); };
@@ -254,7 +260,7 @@ extern "C" int fw_wigner_propagate(fw_wigner_plan* plan, const fw_wigner_desc* d
     ++g_launches;
     if (g_timer) g_timer->mark(0);
     if (totals && a.part_out != nullptr) {
-      e = launch_totals(a.part_out, plan->nparts, M, B, plan->tot, a.obs_hist, st);
+      e = launch_totals(a.part_out, plan->nparts, M, B, plan->tot, a.obs_hist, base.dep, st);
       if (e != cudaSuccess) return cuda_fail(e, "totals launch");
       ++g_launches;
       if (g_timer) g_timer->mark(3);
@@ -299,7 +305,7 @@ extern "C" int fw_wigner_propagate(fw_wigner_plan* plan, const fw_wigner_desc* d
         base.wph = plan->wph;
         base.wph_bs = d->wp_bstride != 0 ? 4LL * plan->P : 0;
         cudaError_t e = launch_pweight_dft(d->wp, d->wp_bstride, d->Mp, plan->P, nb, plan->wph, 4LL * plan->P,
-                                           plan->dtype, st);
+                                           plan->dtype, base.dep, st);
         if (e != cudaSuccess) return cuda_fail(e, "weight spectrum launch");
         ++g_launches;
       }

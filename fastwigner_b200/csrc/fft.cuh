@@ -24,6 +24,14 @@
 
 namespace fw {
 
+// First statement of every pass: wait until the kernels this launch depends on
+// are complete and their memory visible (a no-op without a programmatic
+// dependency), then let the next launch's blocks come up.
+__device__ __forceinline__ void dep_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename R> struct cplx;
 template <> struct cplx<float> { using type = float2; };
 template <> struct cplx<double> { using type = double2; };

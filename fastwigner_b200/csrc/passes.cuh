@@ -74,10 +74,11 @@ struct PassArgs {
   // launch shapes for small batches (RowCfgSmall / ColCfgSmall); decided once
   // per plan, since the row twiddle table and the column record count follow it
   int small_shape;
+  int dep;  // programmatic dependent launch (launch_dep)
 };
 
 // Reduce previous-pass partial sums (per instance) into the input scale.
-// Called by every thread; uses `red` (>= 33 doubles of shared memory).
+// Called by every thread; uses `red` (>= 32 doubles of shared memory).
 __device__ __forceinline__ double prev_scale(const PassArgs& a, int b, double* red, bool first_tile) {
   if (a.prev_tot != nullptr) return 1.0 / (__ldcg(a.prev_tot + (size_t)b * a.M) * a.dxdp);
   if (a.prev_part == nullptr) return a.scale_const;
@@ -91,13 +92,8 @@ __device__ __forceinline__ double prev_scale(const PassArgs& a, int b, double* r
   __syncthreads();
   if ((tid & 31) == 0) red[tid >> 5] = s;
   __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (nth + 31) / 32; ++w) t += red[w];
-    red[32] = t;
-  }
-  __syncthreads();
-  const double tot = red[32];
+  double tot = 0.0;
+  for (int w = 0; w < (nth + 31) / 32; ++w) tot += red[w];  // every thread, the same order
   if (a.obs_hist != nullptr && first_tile) {
     // one warp per column m: lanes sum records lane, lane+32, ...; fixed tree
     double* oh = a.obs_hist + (size_t)b * a.M;

@@ -128,6 +128,7 @@ extern "C" int fw_rho_pass(fw_rho_plan* p, void* R, long long r_bstride, int axi
   for (const fw_rho_factor* f : {f0, f1, f2, f3})
     if (f && f->on && f->shear_c != 0.0) { a.dX = f->shear_dx; a.dP = f->shear_dp; }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  a.dep = dep_launches(st);
   cudaError_t e = axis == 1 ? launch_rho_row(a, p->dtype, st, nullptr) : launch_rho_col(a, p->dtype, st);
   if (e != cudaSuccess) return cuda_fail(e, "fw_rho_pass launch");
   count_launch(1);
@@ -185,6 +186,7 @@ extern "C" int fw_rho_propagate(fw_rho_plan* p, const fw_rho_desc* d, int steps,
   base.Mx = d->Mx;
   base.Mp = d->Mp;
   base.tw = p->tw;
+  base.dep = dep_launches(st);
   const double invN = 1.0 / (double)N;
   int np = 0;
   auto row = [&](RhoArgs a) -> int {

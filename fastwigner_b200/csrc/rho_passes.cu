@@ -47,6 +47,7 @@ struct RhoArgs {
   const double* gp;    // Mp x N complex FP64 (G[(i - j) mod N])
   double* sum_out;     // if non-null: per-CTA complex sum of all elements after F3 (2 doubles)
   const void* tw;
+  int dep;  // programmatic dependent launch (launch_dep)
 };
 
 template <typename Rl>
@@ -178,8 +179,7 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
   __shared__ double red[4];
   __shared__ double ored[G * T / 32][4 + 2 * (2 * RMAXO)];
   const int b = blockIdx.y;
-  double sre, sim;
-  rho_prev_scale(a, b, red, sre, sim);
+  dep_sync();
   const int g = threadIdx.x / T;
   const int j = threadIdx.x % T;
   const int i = blockIdx.x * G + g;
@@ -189,9 +189,14 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
   C* R = reinterpret_cast<C*>(a.R) + (size_t)b * a.r_bs + (size_t)i * N;
   const C* tw = reinterpret_cast<const C*>(a.tw);
   C v[RV];
+  // the loads go out before the scale's reduction
+#pragma unroll
+  for (int m = 0; m < RV; ++m) v[m] = R[j + m * T];
+  double sre, sim;
+  rho_prev_scale(a, b, red, sre, sim);
   const C sc = mk<C>((Rl)sre, (Rl)sim);
 #pragma unroll
-  for (int m = 0; m < RV; ++m) v[m] = cmul(R[j + m * T], sc);
+  for (int m = 0; m < RV; ++m) v[m] = cmul(v[m], sc);
   // The two factor / transform / factor phases run as one loop body (not
   // unrolled): the second phase executes the instructions the first one just
   // fetched, which halves the straight-line code a one-wave launch streams
@@ -301,8 +306,7 @@ __global__ void __launch_bounds__(CP* T, MINB) rho_col_kernel(RhoArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[4];
   const int b = blockIdx.y;
-  double sre, sim;
-  rho_prev_scale(a, b, red, sre, sim);
+  dep_sync();
   const int c = threadIdx.x % CP;
   const int jt = threadIdx.x / CP;
   __builtin_assume(jt >= 0 && jt < T);  // launched with exactly CP * T threads
@@ -312,9 +316,14 @@ __global__ void __launch_bounds__(CP* T, MINB) rho_col_kernel(RhoArgs a) {
   C* R = reinterpret_cast<C*>(a.R) + (size_t)b * a.r_bs;
   const C* tw = reinterpret_cast<const C*>(a.tw);
   C v[RV];
+  // the loads go out before the scale's reduction
+#pragma unroll
+  for (int m = 0; m < RV; ++m) v[m] = R[(size_t)(jt + m * T) * N + col];
+  double sre, sim;
+  rho_prev_scale(a, b, red, sre, sim);
   const C sc = mk<C>((Rl)sre, (Rl)sim);
 #pragma unroll
-  for (int m = 0; m < RV; ++m) v[m] = cmul(R[(size_t)(jt + m * T) * N + col], sc);
+  for (int m = 0; m < RV; ++m) v[m] = cmul(v[m], sc);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f0, jt, col, a.dX, a.dP, b);
   transform<Rl, N, T, RV>(v, a.t1, jt, ex, tw);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f1, jt, col, a.dX, a.dP, b);
@@ -356,8 +365,7 @@ static cudaError_t rho_row_sh(const RhoArgs& a, cudaStream_t st, int* nparts) {
   if (e != cudaSuccess) return e;
   dim3 grid(N / G, a.batch);
   if (nparts) *nparts = grid.x;
-  kern<<<grid, G * T, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, grid, G * T, smem, st, a);
 }
 
 // Passes whose factors shear (the rho -> W transform) use the instantiation
@@ -378,8 +386,7 @@ static cudaError_t rho_col_sh(const RhoArgs& a, cudaStream_t st) {
   cudaError_t e = set_smem_once(attr, kern, smem);
   if (e != cudaSuccess) return e;
   dim3 grid(N / CP, a.batch);
-  kern<<<grid, CP * T, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, grid, CP * T, smem, st, a);
 }
 
 template <typename Rl, int N>

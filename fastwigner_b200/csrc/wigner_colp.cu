@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(CP* T, MINB)
   const int n_items = a.batch * ctl.ntiles;
   const int first = (int)((long long)blockIdx.x * n_items / gridDim.x);
   const int last = (int)((long long)(blockIdx.x + 1) * n_items / gridDim.x);
+  dep_sync();
   if (first >= last) return;  // the same for every thread of the CTA
   const int tid = threadIdx.x;
   constexpr int tab_rowf = 4 * CP;  // floats per table-tile row (complex tables)
@@ -362,9 +363,8 @@ cudaError_t launch_colp_cfg(const PassArgs& a, cudaStream_t st, int* nparts) {
   const int items = a.batch * ntiles;
   const int ctas = sms * S::MINB;
   const int grid = items < ctas ? items : ctas;
-  kern<<<grid, CP * T, L::BYTES, st>>>(mW, mT, a, ctl);
   if (nparts) *nparts = ntiles;
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, grid, CP * T, L::BYTES, st, mW, mT, a, ctl);
 }
 }  // namespace
 

@@ -452,6 +452,7 @@ __global__ void __launch_bounds__(kGenThreads, 2) gen_row_kernel(PassArgs a, Gen
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* z = tw + N;
   C* z2 = z + gen_slot<C>(N << lcp) + 1;
+  dep_sync();
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = __ldg(reinterpret_cast<const C*>(a.tw) + i);
   const Rl s = (Rl)prev_scale(a, b, red, blockIdx.x == 0);
   __syncthreads();
@@ -497,6 +498,7 @@ __global__ void __launch_bounds__(kGenThreads, 2) gen_col_kernel(PassArgs a, Gen
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* z = tw + N;
   C* z2 = z + gen_slot<C>(N << lcp) + 1;
+  dep_sync();
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = __ldg(reinterpret_cast<const C*>(a.tw) + i);
   const Rl s = (Rl)prev_scale(a, b, red, blockIdx.x == 0);
   __syncthreads();
@@ -679,6 +681,7 @@ __global__ void __launch_bounds__(kGenThreads) gen_pweight_kernel(const double* 
   double2* z = tw + P;
   double2* z2 = z + gen_slot<double2>(P) + 1;
   const int q = blockIdx.x, b = blockIdx.y;
+  dep_sync();
   for (int i = threadIdx.x; i < P; i += blockDim.x) {
     double sn, cs;
     sincospi(-2.0 * (double)i / (double)P, &sn, &cs);
@@ -744,15 +747,14 @@ static cudaError_t gen_launch(const PassArgs& a, int dtype, bool row, cudaStream
     static PerDeviceOnce attr;
     cudaError_t e = set_smem_once(attr, gen_row_kernel<Rl>, smem_max);
     if (e != cudaSuccess) return e;
-    gen_row_kernel<Rl><<<dim3(tiles, a.batch), thr, smem, st>>>(a, g, l);
+    return launch_dep(a.dep, gen_row_kernel<Rl>, dim3(tiles, a.batch), thr, smem, st, a, g, l);
   } else {
     static PerDeviceOnce attr;
     cudaError_t e = set_smem_once(attr, gen_col_kernel<Rl>, smem_max);
     if (e != cudaSuccess) return e;
-    gen_col_kernel<Rl><<<dim3(tiles, a.batch), thr, smem, st>>>(a, g, l);
     if (nparts) *nparts = tiles;
+    return launch_dep(a.dep, gen_col_kernel<Rl>, dim3(tiles, a.batch), thr, smem, st, a, g, l);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_generic_row(const PassArgs& a, int dtype, cudaStream_t st) {
@@ -764,20 +766,19 @@ cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, in
 }
 
 cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
-                                   long long out_bs, int dtype, cudaStream_t st) {
+                                   long long out_bs, int dtype, int dep, cudaStream_t st) {
   const GenFactors g = gen_factors(P, false);
   const size_t smem = gen_smem<double2>(P, 0), smem_max = gen_smem<double2>(4096, 0);
   static PerDeviceOnce attr[2];
   if (dtype == FW_F32) {
     cudaError_t e = set_smem_once(attr[0], gen_pweight_kernel<float>, smem_max);
     if (e != cudaSuccess) return e;
-    gen_pweight_kernel<float><<<dim3(Mp, nb), kGenThreads, smem, st>>>(wp, wp_bs, P, out, out_bs, g);
+    return launch_dep(dep, gen_pweight_kernel<float>, dim3(Mp, nb), kGenThreads, smem, st, wp, wp_bs, P, out, out_bs, g);
   } else {
     cudaError_t e = set_smem_once(attr[1], gen_pweight_kernel<double>, smem_max);
     if (e != cudaSuccess) return e;
-    gen_pweight_kernel<double><<<dim3(Mp, nb), kGenThreads, smem, st>>>(wp, wp_bs, P, out, out_bs, g);
+    return launch_dep(dep, gen_pweight_kernel<double>, dim3(Mp, nb), kGenThreads, smem, st, wp, wp_bs, P, out, out_bs, g);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace fw

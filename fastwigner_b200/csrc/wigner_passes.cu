@@ -8,19 +8,21 @@
 #include "fw_internal.h"
 
 namespace fw {
-template <typename Rl, int N, int T, int G, int MINB>
+template <typename Rl, int N, int T, int G, int MINB, bool PAIR>
 __global__ void __launch_bounds__(G* T, MINB) row_pass_kernel(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[34];
-  row_tile<Rl, N, T, G, true>(a, blockIdx.y, blockIdx.x, smem_raw, red);
+  dep_sync();
+  row_tile<Rl, N, T, G, true, PAIR>(a, blockIdx.y, blockIdx.x, smem_raw, red);
 }
 
-template <typename Rl, int N, int T, int CP, int MINB>
+template <typename Rl, int N, int T, int CP, int MINB, bool PAIR>
 __global__ void __launch_bounds__(CP* T, MINB) col_pass_kernel(PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[34];
   __shared__ double ored[(CP * T) / 32][2 + 2 * MAXO];
-  col_tile<Rl, N, T, CP>(a, blockIdx.y, blockIdx.x, gridDim.x, smem_raw, red, ored);
+  dep_sync();
+  col_tile<Rl, N, T, CP, false, PAIR>(a, blockIdx.y, blockIdx.x, gridDim.x, smem_raw, red, ored);
 }
 
 // Per-instance totals of a pass's partial-sum records: block b, warp m < M
@@ -29,6 +31,7 @@ __global__ void __launch_bounds__(CP* T, MINB) col_pass_kernel(PassArgs a) {
 // hist[b*M + m] when hist is set.
 __global__ void totals_kernel(const double* part, int nparts, int M, double* tot, double* hist) {
   const int b = blockIdx.x, m = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  dep_sync();
   if (m >= M) return;  // whole warps
   const double* pp = part + (size_t)b * nparts * M + m;
   double s = 0.0;
@@ -42,9 +45,8 @@ __global__ void totals_kernel(const double* part, int nparts, int M, double* tot
 }
 
 cudaError_t launch_totals(const double* part, int nparts, int M, int batch, double* tot, double* hist,
-                          cudaStream_t st) {
-  totals_kernel<<<batch, 32 * M, 0, st>>>(part, nparts, M, tot, hist);
-  return cudaGetLastError();
+                          int dep, cudaStream_t st) {
+  return launch_dep(dep, totals_kernel, batch, 32 * M, 0, st, part, nparts, M, tot, hist);
 }
 
 // ---------------------------------------------------------------------------
@@ -54,6 +56,7 @@ template <typename Rl>
 __global__ void finalize_kernel(PassArgs a, int vec) {
   __shared__ double red[34];
   const int b = blockIdx.y;
+  dep_sync();
   const double sc = prev_scale(a, b, red, blockIdx.x == 0);
   Rl* W = reinterpret_cast<Rl*>(a.W) + (size_t)b * a.w_bs;
   const size_t n = (size_t)a.P * a.X;
@@ -137,49 +140,47 @@ template <> struct RowCfgSmall<float, 2048> { static constexpr int T = 64, G = 1
 
 constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
 
-template <typename Rl, int N, int T, int G, int MINB>
+template <typename Rl, int N, int T, int G, int MINB, bool PAIR>
 static cudaError_t launch_row_cfg(const PassArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)G * 2 * (N + N / 32) * sizeof(Rl);
-  auto kern = row_pass_kernel<Rl, N, T, G, MINB>;
+  auto kern = row_pass_kernel<Rl, N, T, G, MINB, PAIR>;
   static PerDeviceOnce attr;  // per device: the attribute is set on the device current at the call
   cudaError_t e = set_smem_once(attr, kern, smem);
   if (e != cudaSuccess) return e;
   dim3 grid((a.P / 2 + G - 1) / G, a.batch);
-  kern<<<grid, G * T, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, grid, G * T, smem, st, a);
 }
 
 template <typename Rl, int N>
 static cudaError_t launch_row_n(const PassArgs& a, cudaStream_t st) {
   if (a.small_shape) {
     using Cfg = RowCfgSmall<Rl, N>;
-    return launch_row_cfg<Rl, N, Cfg::T, Cfg::G, Cfg::MINB>(a, st);
+    return launch_row_cfg<Rl, N, Cfg::T, Cfg::G, Cfg::MINB, sizeof(Rl) == 8>(a, st);  // (FP32: spectral_mul_bins)
   }
   using Cfg = RowCfg<Rl, N>;
-  return launch_row_cfg<Rl, N, Cfg::T, Cfg::G, Cfg::MINB>(a, st);
+  return launch_row_cfg<Rl, N, Cfg::T, Cfg::G, Cfg::MINB, true>(a, st);
 }
 
-template <typename Rl, int N, int T, int CP, int MINB>
+template <typename Rl, int N, int T, int CP, int MINB, bool PAIR>
 static cudaError_t launch_col_cfg(const PassArgs& a, cudaStream_t st, int* nparts) {
   const size_t smem = col_smem_bytes<Rl, N, T, CP>();
-  auto kern = col_pass_kernel<Rl, N, T, CP, MINB>;
+  auto kern = col_pass_kernel<Rl, N, T, CP, MINB, PAIR>;
   static PerDeviceOnce attr;  // per device: the attribute is set on the device current at the call
   cudaError_t e = set_smem_once(attr, kern, smem);
   if (e != cudaSuccess) return e;
   dim3 grid(a.X / (2 * CP), a.batch);
   if (nparts) *nparts = grid.x;
-  kern<<<grid, CP * T, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, grid, CP * T, smem, st, a);
 }
 
 template <typename Rl, int N>
 static cudaError_t launch_col_n(const PassArgs& a, cudaStream_t st, int* nparts) {
   if (a.small_shape) {
     using Cfg = ColCfgSmall<Rl, N>;
-    return launch_col_cfg<Rl, N, Cfg::T, Cfg::CP, Cfg::MINB>(a, st, nparts);
+    return launch_col_cfg<Rl, N, Cfg::T, Cfg::CP, Cfg::MINB, sizeof(Rl) == 8>(a, st, nparts);
   }
   using Cfg = ColCfg<Rl, N>;
-  return launch_col_cfg<Rl, N, Cfg::T, Cfg::CP, Cfg::MINB>(a, st, nparts);
+  return launch_col_cfg<Rl, N, Cfg::T, Cfg::CP, Cfg::MINB, true>(a, st, nparts);
 }
 
 // Column passes of sizes the register-resident kernels do not take (P not a
@@ -277,9 +278,7 @@ cudaError_t launch_finalize(const PassArgs& a, int dtype, cudaStream_t st) {
   if (blocks > need) blocks = need;
   if (blocks < 1) blocks = 1;
   dim3 grid((unsigned)blocks, a.batch);
-  if (dtype == FW_F32) finalize_kernel<float><<<grid, 256, 0, st>>>(a, vec);
-  else finalize_kernel<double><<<grid, 256, 0, st>>>(a, vec);
-  return cudaGetLastError();
+  return launch_dep(a.dep, dtype == FW_F32 ? finalize_kernel<float> : finalize_kernel<double>, grid, 256, 0, st, a, vec);
 }
 
 // Forward DFT Wh[k] = sum_p w[p] exp(-2 pi i k p / P) of each p-observable
@@ -293,6 +292,7 @@ __global__ void __launch_bounds__(256) pweight_dft_kernel(const double* wp, long
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* x = reinterpret_cast<double2*>(smem_raw);
   double2* y = x + P;
+  dep_sync();
   const int q = blockIdx.x, b = blockIdx.y;
   const double* w = wp + (size_t)b * wp_bs + (size_t)q * P;
   for (int i = threadIdx.x; i < P; i += blockDim.x) x[i] = make_double2(w[i], 0.0);
@@ -319,21 +319,21 @@ __global__ void __launch_bounds__(256) pweight_dft_kernel(const double* wp, long
 }
 
 cudaError_t launch_pweight_dft(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out, long long out_bs,
-                               int dtype, cudaStream_t st) {
-  if (!is_pow2(P)) return launch_generic_pweight(wp, wp_bs, Mp, P, nb, out, out_bs, dtype, st);
+                               int dtype, int dep, cudaStream_t st) {
+  if (!is_pow2(P)) return launch_generic_pweight(wp, wp_bs, Mp, P, nb, out, out_bs, dtype, dep, st);
   const size_t smem = 2 * sizeof(double2) * (size_t)P;
   dim3 grid(Mp, nb);
   cudaError_t e;
   if (dtype == FW_F32) {
     e = cudaFuncSetAttribute(pweight_dft_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    pweight_dft_kernel<float><<<grid, 256, smem, st>>>(wp, wp_bs, P, out, out_bs);
+    e = launch_dep(dep, pweight_dft_kernel<float>, grid, 256, smem, st, wp, wp_bs, P, out, out_bs);
   } else {
     e = cudaFuncSetAttribute(pweight_dft_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    pweight_dft_kernel<double><<<grid, 256, smem, st>>>(wp, wp_bs, P, out, out_bs);
+    e = launch_dep(dep, pweight_dft_kernel<double>, grid, 256, smem, st, wp, wp_bs, P, out, out_bs);
   }
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fw

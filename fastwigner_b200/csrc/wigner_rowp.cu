@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 1) row_persist_kernel(PassArgs
   C* Ts = reinterpret_cast<C*>(mine + L::W_BYTES);
   C* exz = reinterpret_cast<C*>(mine + L::W_BYTES + L::T_BYTES);
   C* tws = reinterpret_cast<C*>(smem + (size_t)kRowWarps * L::WARP_BYTES);
+  dep_sync();
   for (int i = threadIdx.x; i < L::STW; i += blockDim.x) tws[i] = reinterpret_cast<const C*>(a.tw)[i];
   if (lane == 0) {
     mbar_init(&bars[w][0], 1);
@@ -179,8 +180,7 @@ cudaError_t launch_row_persist(const PassArgs& a, cudaStream_t st) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int npairs = a.P / 2;
-  kern<<<sms, 32 * kRowWarps, L::BYTES, st>>>(a, npairs);
-  return cudaGetLastError();
+  return launch_dep(a.dep, kern, sms, 32 * kRowWarps, L::BYTES, st, a, npairs);
 }
 
 }  // namespace fw

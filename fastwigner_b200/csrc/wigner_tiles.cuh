@@ -147,19 +147,56 @@ __device__ __forceinline__ void spectral_mul(cplx_t<Rl> (&v)[RV], const int j, E
   ex.sync();
 }
 
+// The same multiply bin by bin, for the FP32 passes of few blocks (one object
+// of the drop-in classes).  Its sums round differently from pair_mid's, and the
+// observables of one FP32 object on a wide box (x to 200 in the strong-field
+// runs) carry that rounding at 1e-5 of their value: they stay what they were.
+// Those launches are bound by latency; the paired form gained them under 5 %.
+template <typename Rl, int N, int T, int RV, typename EX>
+__device__ __forceinline__ void spectral_mul_bins(cplx_t<Rl> (&v)[RV], const int j, EX& ex, const void* taba,
+                                                  const void* tabb, size_t tab_stride, int tab_real, const void* g,
+                                                  Rl f) {
+  using C = cplx_t<Rl>;
+  ex_write_natural<T, RV>(ex, j, v);
+  ex.sync();
+  constexpr bool kFoldMirror = EX::kFold && T % (1 << EX::kL) == 0;
+  const int mbase = kFoldMirror ? ex.map(N - j) : 0;  // virtual slot of N for j = 0
+#pragma unroll
+  for (int m = 0; m < RV; ++m) {
+    const int k = j + m * T;
+    const int kk = (k <= N / 2) ? k : N - k;
+    C ea = tab_load<Rl>(taba, tab_real, (size_t)kk * tab_stride), eb = tab_load<Rl>(tabb, tab_real, (size_t)kk * tab_stride);
+    if (g != nullptr) {
+      const C gk = __ldg(reinterpret_cast<const C*>(g) + kk);
+      ea = cmul(ea, gk);
+      eb = cmul(eb, gk);
+    }
+    ea = herm(ea, k, N);
+    eb = herm(eb, k, N);
+    C znk;
+    if constexpr (kFoldMirror) {
+      znk = ex.read_at(m == 0 ? (j == 0 ? ex.map(0) : mbase) : mbase - EX::delta(m * T));
+    } else {
+      znk = ex.read((N - k) & (N - 1));
+    }
+    v[m] = two_real_mul(v[m], znk, ea, eb, f);
+  }
+  ex.sync();
+}
+
 // ---------------------------------------------------------------------------
 // Row pass: G groups of T threads, each group owns one pair of rows.
 // One CTA-sized work item of a row pass: instance b, row pairs blk*G .. blk*G+G-1.
 // STW: a.tw is the stage-layout twiddle table of (N, N/T) instead of exp(-2 pi i k/N).
-template <typename Rl, int N, int T, int G, bool STW = false>
+// PAIR: the paired spectral multiply.
+template <typename Rl, int N, int T, int G, bool STW = false, bool PAIR = true>
 __device__ __forceinline__ void row_tile(const PassArgs& a, int b, int blk, unsigned char* smem_raw, double* red) {
   using C = cplx_t<Rl>;
   constexpr int RV = N / T;
-  const double sc = prev_scale(a, b, red, blk == 0);
   const int g = threadIdx.x / T;
   const int j = threadIdx.x % T;
   const int rp = blk * G + g;
-  if (2 * rp >= a.P) return;  // group-scoped synchronisation only below
+  const bool in = 2 * rp < a.P;
   constexpr int BUF = N + N / 32;
   Rl* base = reinterpret_cast<Rl*>(smem_raw) + (size_t)g * 2 * BUF;
   GroupEx<Rl, T> ex{base, base + BUF, 1 + g};
@@ -167,18 +204,25 @@ __device__ __forceinline__ void row_tile(const PassArgs& a, int b, int blk, unsi
   Rl* W = reinterpret_cast<Rl*>(a.W) + (size_t)b * a.w_bs + (size_t)(2 * rp) * N;
   const C* tw = reinterpret_cast<const C*>(a.tw);
   C v[RV];
-  const Rl s = (Rl)sc;
+  // the loads go out before the scale's reduction
+  if (in) {
 #pragma unroll
-  for (int m = 0; m < RV; ++m) {
-    const int x = j + m * T;
-    v[m] = mk<C>(__ldcg(W + x) * s, __ldcg(W + N + x) * s);
+    for (int m = 0; m < RV; ++m) {
+      const int x = j + m * T;
+      v[m] = mk<C>(__ldcg(W + x), __ldcg(W + N + x));
+    }
   }
+  const Rl s = (Rl)prev_scale(a, b, red, blk == 0);
+  if (!in) return;  // group-scoped synchronisation only below
+#pragma unroll
+  for (int m = 0; m < RV; ++m) v[m] = cscale(v[m], s);
   fft<N, T, RV, -1, C, EXT, STW>(v, j, ex, tw);
   const size_t esz = a.tab_real ? sizeof(Rl) : sizeof(C);
   const size_t hs = N / 2 + 1;
   const char* tb = reinterpret_cast<const char*>(a.tab1) + ((size_t)b * a.tab_bs + (size_t)(2 * rp) * hs) * esz;
   const Rl f = (Rl)(a.out_scale / (double)N);
-  spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + hs * esz, 1, a.tab_real, a.g1, f);
+  if constexpr (PAIR) spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + hs * esz, 1, a.tab_real, a.g1, f);
+  else spectral_mul_bins<Rl, N, T, RV>(v, j, ex, tb, tb + hs * esz, 1, a.tab_real, a.g1, f);
   fft<N, T, RV, +1, C, EXT, STW>(v, j, ex, tw);
 #pragma unroll
   for (int m = 0; m < RV; ++m) {
@@ -205,14 +249,35 @@ template <> struct Vec2<double> { using type = double2; };
 template <int NTHR>
 __device__ __forceinline__ void obs_store(const PassArgs& a, int b, int tile, int ntiles, double (&acc)[2 + 2 * MAXO],
                                           double (*ored)[2 + 2 * MAXO]) {
+  // reduce-scatter over the warp: at each of the first three levels a lane
+  // keeps half of its (padded) values and sends the other half, so ten sums cost
+  // 8 + 4 + 2 + 2 x 2 shuffles of a double instead of 10 x 5; lane l ends with the
+  // sums of values 2 (l >> 2) and 2 (l >> 2) + 1
+  constexpr int NV = 2 + 2 * MAXO;
+  static_assert(NV <= 16, "values per record");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double u[16];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)  // level-major: the accumulators reduce in parallel
+  for (int q = 0; q < 16; ++q) u[q] = q < NV ? acc[q < NV ? q : 0] : 0.0;
 #pragma unroll
-    for (int q = 0; q < 2 + 2 * MAXO; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
+  for (int lv = 0; lv < 3; ++lv) {
+    const int off = 16 >> lv, half = 8 >> lv;
+    const bool up = (lane & off) != 0;
 #pragma unroll
-    for (int q = 0; q < 2 + 2 * MAXO; ++q) ored[warp][q] = acc[q];
+    for (int q = 0; q < half; ++q) {
+      const double send = up ? u[q] : u[q + half], keep = up ? u[q + half] : u[q];
+      u[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    u[0] += __shfl_xor_sync(0xffffffffu, u[0], o);
+    u[1] += __shfl_xor_sync(0xffffffffu, u[1], o);
+  }
+  if ((lane & 3) == 0) {
+    const int q = 2 * (lane >> 2);
+    if (q < NV) ored[warp][q] = u[0];
+    if (q + 1 < NV) ored[warp][q + 1] = u[1];
   }
   __syncthreads();
   if (threadIdx.x < a.M) {
@@ -472,13 +537,12 @@ template <typename Rl, int N, int T, int CP> constexpr size_t col_smem_bytes() {
   return (col_ex_reals<Rl, N, T, CP>() + (size_t)2 * N) * sizeof(Rl);
 }
 
-template <typename Rl, int N, int T, int CP, bool STW = false>
+template <typename Rl, int N, int T, int CP, bool STW = false, bool PAIR = true>
 __device__ __forceinline__ void col_tile(const PassArgs& a, int b, int tile, int ntiles, unsigned char* smem_raw,
                                          double* red, double (*ored)[2 + 2 * MAXO]) {
   using C = cplx_t<Rl>;
   using V2 = typename Vec2<Rl>::type;
   constexpr int RV = N / T;
-  const double sc = prev_scale(a, b, red, tile == 0);
   const int c = threadIdx.x % CP;
   const int j = threadIdx.x / CP;
   // every launch of a column tile has exactly CP * T threads; telling the
@@ -492,13 +556,16 @@ __device__ __forceinline__ void col_tile(const PassArgs& a, int b, int tile, int
   Rl* W = reinterpret_cast<Rl*>(a.W) + (size_t)b * a.w_bs;
   const C* tw = reinterpret_cast<const C*>(a.tw);
   C v[RV];
-  const Rl s = (Rl)sc;
+  // the loads go out before the scale's reduction
 #pragma unroll
   for (int m = 0; m < RV; ++m) {
     const int p = j + m * T;
     const V2 w = __ldcg(reinterpret_cast<const V2*>(W + (size_t)p * X + xa));
-    v[m] = mk<C>(w.x * s, w.y * s);
+    v[m] = mk<C>(w.x, w.y);
   }
+  const Rl s = (Rl)prev_scale(a, b, red, tile == 0);
+#pragma unroll
+  for (int m = 0; m < RV; ++m) v[m] = cscale(v[m], s);
   if (a.blend_pre) {
     const Rl* S0 = reinterpret_cast<const Rl*>(a.s0) + (size_t)b * a.s0_bs;
     const Rl bc = (Rl)a.blend_c;
@@ -524,7 +591,8 @@ __device__ __forceinline__ void col_tile(const PassArgs& a, int b, int tile, int
   if (a.tab1 != nullptr) {
     fft<N, T, RV, -1, C, EXT, STW>(v, j, ex, tw);
     const char* tb = reinterpret_cast<const char*>(a.tab1) + ((size_t)b * a.tab_bs + xa) * esz;
-    spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g1, f);
+    if constexpr (PAIR) spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g1, f);
+    else spectral_mul_bins<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g1, f);
     fft<N, T, RV, +1, C, EXT, STW>(v, j, ex, tw);
   }
   if (a.bxp != nullptr) {
@@ -554,39 +622,38 @@ __device__ __forceinline__ void col_tile(const PassArgs& a, int b, int tile, int
     const double* wp = a.wp + (size_t)b * a.wp_bs;
     const int P = N;
     if constexpr (sizeof(Rl) == 4) {
-      // FP32 state: the 2*CP columns of a row sit in CP adjacent lanes; reduce a
-      // row's sums across them with shuffles (log2 CP additions), then one lane
-      // per row accumulates the FP64 weighted sums; the per-thread column sums
+      // FP32 state: the 2*CP columns of a row sit in CP adjacent lanes; their
+      // sums reduce across them by recursive halving (at each level a lane keeps
+      // half of the rows and sends the other half), which leaves every lane NB/CP
+      // rows whose FP64 weighted sums it accumulates; the per-thread column sums
       // over RV rows accumulate in FP64.
       double fa = 0.0, fb = 0.0;
-      constexpr int CH = RV < 8 ? RV : 8;  // rows per batch of independent shuffles
+      constexpr int NB = RV < CP ? CP : (RV < 8 ? RV : (CP > 8 ? CP : 8));  // rows of a block (a multiple of CP)
 #pragma unroll
-      for (int m0 = 0; m0 < RV; m0 += CH) {
-        float s[CH], s2[CH];
+      for (int m0 = 0; m0 < RV; m0 += NB) {
+        C u[NB];  // (sum, sum of squares) of a row's pair; rows past RV are zero
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-          const float wa = v[m0 + u].x, wb = v[m0 + u].y;
-          fa += wa;
-          fb += wb;
-          s[u] = wa + wb;
-          s2[u] = wa * wa + wb * wb;
-        }
-#pragma unroll
-        for (int o = CP / 2; o >= 1; o >>= 1)
-#pragma unroll
-          for (int u = 0; u < CH; ++u) {  // level-major: CH independent shuffles in flight
-            s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-            s2[u] += __shfl_xor_sync(0xffffffffu, s2[u], o);
+        for (int i = 0; i < NB; ++i) {
+          if (m0 + i < RV) {
+            const float wa = v[m0 + i < RV ? m0 + i : 0].x, wb = v[m0 + i < RV ? m0 + i : 0].y;
+            fa += wa;
+            fb += wb;
+            u[i] = mk<C>(wa + wb, wa * wa + wb * wb);
+          } else {
+            u[i] = mk<C>(0.f, 0.f);
           }
-        if (c == 0) {
+        }
+        halving_sum<CP, NB>(u, c);  // lane c: rows m0 + c NB/CP + i
 #pragma unroll
-          for (int u = 0; u < CH; ++u) {
-            const int p = j + (m0 + u) * T;
-            acc[0] += (double)s[u];
-            acc[1] += (double)s2[u];
+        for (int i = 0; i < NB / CP; ++i) {
+          const int m = m0 + c * (NB / CP) + i;
+          if (m < RV) {
+            const int p = j + m * T;
+            acc[0] += (double)u[i].x;
+            acc[1] += (double)u[i].y;
 #pragma unroll
             for (int q = 0; q < MAXO; ++q)
-              if (q < a.Mp) acc[2 + MAXO + q] += (double)s[u] * __ldg(wp + (size_t)q * P + p);
+              if (q < a.Mp) acc[2 + MAXO + q] += (double)u[i].x * __ldg(wp + (size_t)q * P + p);
           }
         }
       }
@@ -615,7 +682,8 @@ __device__ __forceinline__ void col_tile(const PassArgs& a, int b, int tile, int
   if (a.tab2 != nullptr) {
     fft<N, T, RV, -1, C, EXT, STW>(v, j, ex, tw);
     const char* tb = reinterpret_cast<const char*>(a.tab2) + ((size_t)b * a.tab_bs + xa) * esz;
-    spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g2, f);
+    if constexpr (PAIR) spectral_mul<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g2, f);
+    else spectral_mul_bins<Rl, N, T, RV>(v, j, ex, tb, tb + esz, (size_t)X, a.tab_real, a.g2, f);
     fft<N, T, RV, +1, C, EXT, STW>(v, j, ex, tw);
   }
   col_store<Rl, N, T, RV>(a, v, W, j, xa);
