@@ -90,7 +90,9 @@ struct LayerArgs {
   float* fx;           // [tile][rows][32 o][32 k]
   const float *Q1, *c1, *Q2, *c2;  // LAST
   float* out;          // LAST: [rows][G1]
-  int rows, G1, tiles, act;
+  int rows, G1, tiles, act;  // act: 0 none, 1 GELU, 2 times GELU'(aux)
+  const float* aux;     // channel-major [b][32][G0][G1], as the three below; LIFT: v' is read from it instead
+  float *pre, *vcm;     // optional copies of the pre-activation and of v'
 };
 
 // float index of element (row, k) of a 128-byte-row, 128-byte-swizzled tile
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
   const int nx = min(LX, a.G1 - x0);
   const int ncta = (gridDim.x - tile + a.tiles - 1) / a.tiles;  // CTAs of this x tile
   const int stride = 2 * ncta;
+  const bool next = MODE != LAYER_LAST && a.fx != nullptr;  // v' goes on: pixel-major copy and x-transform
 
   if (tid < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       Wl[sw(i >> 5, i & 31)] = l;
     }
   }
-  if (MODE != LAYER_LAST) {
+  if (next) {
     // 4 chunks of 32 pixels: rows 0-31 the modes' high parts, 32-63 the low parts
     for (int i = tid; i < LX * LK; i += 256) {
       const int x = i >> 5, k = i & 31;
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       CSs[(x >> 5) * 2048 + sw(k, x & 31)] = h;
       CSs[(x >> 5) * 2048 + sw(32 + k, x & 31)] = l;
     }
-  } else {
+  } else if (MODE == LAYER_LAST) {
     for (int i = tid; i < PROJ * LC; i += 256) {
       float h, l;
       split_tf32(__ldg(a.Q1 + i), h, l);
@@ -179,9 +182,9 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       s_q2[tid] = __ldg(a.Q2 + tid);
     }
   }
-  if (tid < LC) s_bias[tid] = __ldg(a.bias + tid);
+  if (tid < LC) s_bias[tid] = a.bias != nullptr ? __ldg(a.bias + tid) : 0.f;
   float* s_w0 = AAh;  // LIFT: the input weights, input-major, in the unused DFT tile
-  if constexpr (MODE == LAYER_LIFT)
+  if (MODE == LAYER_LIFT && a.aux == nullptr)
     for (int i = tid; i < LC * (a.NP + 2); i += 256) s_w0[(i % (a.NP + 2)) * LC + i / (a.NP + 2)] = __ldg(a.W + i);
   unsigned char* mine = sm + S_SLOT + slot * T_BYTES;
   // pixels past the row's end are never loaded: keep their buffer rows finite
@@ -199,6 +202,11 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
   const uint32_t aAAh = smem_u32(AAh), aAAl = smem_u32(AAl), aCS = smem_u32(CSs), aW = smem_u32(Wh);
   uint64_t* bar = bars[slot];
   const uint32_t vbytes = (uint32_t)nx * LC * 4;
+  const size_t chs = (size_t)a.G0 * a.G1;                     // channel stride of the channel-major arrays
+  auto cm_base = [&](int r) {                                 // this thread's pixel of row r, channel 0
+    const int b = r / a.G0;
+    return ((size_t)b * LC * a.G0 + (r - b * a.G0)) * a.G1 + x0 + st;
+  };
   auto slot_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory"); };
   auto load_v = [&](int r, int buf) {  // one thread of the slot
     mbar_arrive_expect_tx(&bar[buf], vbytes);
@@ -317,27 +325,57 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       tmem_ld64(trow + D1_COL + 64, t);
 #pragma unroll
       for (int i = 0; i < LC; ++i) v[i] = v[i] + (t[i] + t[32 + i]) + s_bias[i];
-      if (a.act) {
+      if (MODE == LAYER_MID && a.pre != nullptr && st < nx) {
+        float* p = a.pre + cm_base(r);
+#pragma unroll
+        for (int i = 0; i < LC; ++i) p[i * chs] = v[i];
+      }
+      if (a.act == 1) {
 #pragma unroll
         for (int i = 0; i < LC; i += 2) gelu2(v[i], v[i + 1]);
+      } else if (MODE == LAYER_MID && a.act == 2) {
+        const float* p = a.aux + cm_base(r);
+#pragma unroll
+        for (int h = 0; h < LC; h += 16) {
+          float x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = st < nx ? __ldg(p + (h + i) * chs) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[h + i] *= gelu_d(x[i]);
+        }
       }
     } else {
       if (d2_prev) store_d2();
       if (warp == 0 && elect_lane()) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the buffers alternate
-      if (warp == 1) {  // the row's constant part, a channel per lane
+      if (a.aux == nullptr && warp == 1) {  // the row's constant part, a channel per lane
         const int b = r / a.G0;
         float c = s_bias[lane] + s_w0[(a.NP + 1) * LC + lane] * __ldg(a.ps + (r - b * a.G0));
         for (int q = 0; q < a.NP; ++q) c += s_w0[q * LC + lane] * __ldg(a.par + (size_t)b * a.NP + q);
         s_row[slot][lane] = c;
       }
       slot_sync();  // the outgoing copy of this buffer has been read
-      const float x = st < nx ? __ldg(a.xs + x0 + st) : 0.f;
+      if (a.aux != nullptr) {
+        const float* p = a.aux + cm_base(r);
 #pragma unroll
-      for (int i = 0; i < LC; ++i) v[i] = s_row[slot][i] + s_w0[a.NP * LC + i] * x;
+        for (int i = 0; i < LC; ++i) v[i] = st < nx ? __ldg(p + i * chs) : 0.f;
+      } else {
+        const float x = st < nx ? __ldg(a.xs + x0 + st) : 0.f;
+#pragma unroll
+        for (int i = 0; i < LC; ++i) v[i] = s_row[slot][i] + s_w0[a.NP * LC + i] * x;
+      }
     }
     if (st >= nx) {
 #pragma unroll
       for (int i = 0; i < LC; ++i) v[i] = 0.f;
+    }
+    if (MODE != LAYER_LAST && a.vcm != nullptr && st < nx) {
+      float* p = a.vcm + cm_base(r);
+#pragma unroll
+      for (int i = 0; i < LC; ++i) p[i * chs] = v[i];
+    }
+    if (MODE != LAYER_LAST && !next) {  // nothing on the chip follows
+      buf ^= 1;
+      continue;
     }
     if (MODE != LAYER_LAST) {
       // v' as a pixel row for the outgoing copy, and transposed (channel rows
@@ -667,22 +705,29 @@ using namespace fw::fnol;
 extern "C" int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float* gx, const float* AA,
                             const float* CS, const float* W, const float* bias, int act, int NP, const float* par,
                             const float* xs, const float* ps, const float* Q1, const float* c1, const float* Q2, const float* c2,
-                            float* vout, float* fx, float* out, void* stream) {
+                            float* vout, float* fx, float* out, const float* aux, float* pre, float* vcm,
+                            void* stream) {
   if (int rc = check_dims(B, G0, G1, "fw_fno_layer")) return rc;
   if (mode < LAYER_LIFT || mode > LAYER_LAST) return fail(FW_EINVAL, "fw_fno_layer: mode must be 0, 1 or 2");
-  if (bias == nullptr || W == nullptr) return fail(FW_EINVAL, "fw_fno_layer: NULL weights");
+  const bool copy = mode == LAYER_LIFT && aux != nullptr;
+  if (!copy && (W == nullptr || (bias == nullptr && mode != LAYER_MID)))
+    return fail(FW_EINVAL, "fw_fno_layer: NULL weights");
   if (mode == LAYER_LIFT && (NP < 0 || NP > kMaxParams)) return fail(FW_EINVAL, "fw_fno_layer: NP must be in [0, 14]");
-  if (mode == LAYER_LIFT ? ((NP > 0 && par == nullptr) || xs == nullptr || ps == nullptr)
+  if (act < 0 || act > 2 || (act == 2 && (mode != LAYER_MID || aux == nullptr)))
+    return fail(FW_EINVAL, "fw_fno_layer: act must be 0, 1 or (mode 1, with aux) 2");
+  if (mode == LAYER_LIFT ? (!copy && ((NP > 0 && par == nullptr) || xs == nullptr || ps == nullptr))
                          : (!on16(vin) || !on16(gx) || AA == nullptr))
     return fail(FW_EINVAL, "fw_fno_layer: NULL input, or activations off 16 bytes");
   if (mode == LAYER_LAST ? (Q1 == nullptr || c1 == nullptr || Q2 == nullptr || c2 == nullptr || out == nullptr)
-                         : (!on16(vout) || CS == nullptr || fx == nullptr))
+      : fx == nullptr    ? (vcm == nullptr || vout != nullptr)
+                         : (!on16(vout) || CS == nullptr))
     return fail(FW_EINVAL, "fw_fno_layer: NULL output, or activations off 16 bytes");
   LayerArgs a{};
   a.vin = vin, a.gx = gx, a.AA = AA, a.CS = CS, a.W = W, a.bias = bias, a.act = act;
   a.NP = NP, a.par = par, a.xs = xs, a.ps = ps, a.G0 = G0;
   if (int rc = fno_status_ptr(&a.status)) return rc;
   a.vout = vout, a.fx = fx, a.Q1 = Q1, a.c1 = c1, a.Q2 = Q2, a.c2 = c2, a.out = out;
+  a.aux = aux, a.pre = pre, a.vcm = vcm;
   a.rows = B * G0, a.G1 = G1, a.tiles = (G1 + LX - 1) / LX;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = mode == LAYER_LIFT  ? launch_layer<LAYER_LIFT>(a, st)

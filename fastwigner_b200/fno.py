@@ -73,11 +73,11 @@ class _Ops:
                                       stream_handle()), "fw_fno_project")
 
     def layer(self, mode, B, G0, G1, W, bias, act=0, vin=None, gx=None, AA=None, CS=None, NP=0, par=None, xs=None,
-              ps=None, Q1=None, c1=None, Q2=None, c2=None, vout=None, fx=None, out=None):
+              ps=None, Q1=None, c1=None, Q2=None, c2=None, vout=None, fx=None, out=None, aux=None, pre=None, vcm=None):
         opt = lambda t: _p(t) if t is not None else None
-        check(self.lib.fw_fno_layer(mode, B, G0, G1, opt(vin), opt(gx), opt(AA), opt(CS), _p(W), _p(bias), int(act),
+        check(self.lib.fw_fno_layer(mode, B, G0, G1, opt(vin), opt(gx), opt(AA), opt(CS), opt(W), opt(bias), int(act),
                                     NP, opt(par), opt(xs), opt(ps), opt(Q1), opt(c1), opt(Q2), opt(c2), opt(vout),
-                                    opt(fx), opt(out), stream_handle()), "fw_fno_layer")
+                                    opt(fx), opt(out), opt(aux), opt(pre), opt(vcm), stream_handle()), "fw_fno_layer")
 
     def thermal(self, out, wc, xs, ps, x_e, dxdp):
         """Thermal states from network outputs (in place), see fw_fno_thermal."""
@@ -229,12 +229,16 @@ class FNO2d:
         feats = torch.empty((B, NP + 2, G0, G1), dtype=torch.float32, device=dev)
         o.features(B, NP, G0, G1, pr, xs_t, ps_t, feats)
         v = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
-        o.gemm_ex(0, 0, C, L, NP + 2, P["W0"], NP + 2, 0, feats, L, (NP + 2) * L, v, L, C * L, B, bias=P["b0"])
-        c = {"B": B, "G0": G0, "G1": G1, "feats": feats, "v": [], "F2": [], "pre": []}
+        c = {"B": B, "G0": G0, "G1": G1, "feats": feats, "v": [], "F2": [], "pre": [], "lift": (pr, xs_t, ps_t)}
+        if not self._fused_layers(G0, G1):
+            o.gemm_ex(0, 0, C, L, NP + 2, P["W0"], NP + 2, 0, feats, L, (NP + 2) * L, v, L, C * L, B, bias=P["b0"])
         Kp, mx, K = self.Kp, self.mx, self.K
-        Fx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev)
-        Gx = torch.empty_like(Fx)
-        for l in range(self.layers):
+        fused = self._fused_layers(G0, G1)
+        if fused:
+            v = self._layers_cached(c, v, CS, Dpv, Dpiv, AA)
+        Fx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev) if not fused else None
+        Gx = torch.empty_like(Fx) if not fused else None
+        for l in range(0 if fused else self.layers):
             if cache:
                 c["v"].append(v)
             # truncated forward DFT: x (cosine and sine parts in one product), then p
@@ -277,6 +281,67 @@ class FNO2d:
         the surrogate's own width, modes and projection on any grid they hold."""
         return (self.C == 32 and self.mp == self.mx == 16 and self.proj == 128 and self.layers >= 1
                 and self.NP <= 14 and 32 <= G0 <= 1024 and G1 >= 32 and G1 % 4 == 0)
+
+    def _layers_cached(self, c, v, CS, Dpv, Dpiv, AA):
+        """The lift (into v) and the layers by the fused kernels, keeping for the
+        backward pass what the unfused ones keep; returns the last layer's output."""
+        o, P, dev, C, K = self.ops, self.params, self.device, self.C, self.K
+        B, G0, G1 = c["B"], c["G0"], c["G1"]
+        pr, xs_t, ps_t = c["lift"]
+        vp = torch.empty((B, G0, G1, C), dtype=torch.float32, device=dev)
+        fx = torch.empty(((G1 + 127) // 128, B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        gx = torch.empty((B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        O2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)
+        o.layer(0, B, G0, G1, P["W0"], P["b0"], CS=CS, NP=self.NP, par=pr, xs=xs_t, ps=ps_t, vout=vp, fx=fx, vcm=v)
+        for l in range(self.layers):
+            c["v"].append(v)
+            F2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)
+            o.pdft(B, G0, G1, fx, Dpv, F2)
+            c["F2"].append(F2)
+            o.mix(0, B, C, C, K, F2, P[f"R{l}"], O2)
+            o.pidft(B, G0, O2, Dpiv, gx)
+            v = torch.empty_like(v)
+            last = l == self.layers - 1
+            pre = None if last else torch.empty_like(v)
+            o.layer(1, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], act=int(not last), vin=vp, gx=gx, AA=AA, CS=CS,
+                    vout=None if last else vp, fx=None if last else fx, pre=pre, vcm=v)
+            c["pre"].append(pre)
+        return v
+
+    def _transposed(self, G0, G1):
+        """The DFT matrices of _grid transposed, for the fused backward layers."""
+        key = (G0, G1, "T")
+        if key not in self._mats:
+            self._mats[key] = [m.t().contiguous() for m in self._grid(G0, G1)]
+        return self._mats[key]
+
+    def _layers_backward(self, dv, c):
+        """Gradients of the layers from dv, the gradient of the last layer's output
+        (channel-major): each layer's input gradient, times GELU' of the layer
+        below, and its transform in one pass.  Returns the lift's gradient."""
+        o, P, g, dev = self.ops, self.params, self.grads, self.device
+        B, G0, G1, C, K = c["B"], c["G0"], c["G1"], self.C, self.K
+        L = G0 * G1
+        CST, DpvT, DpivT, AAT = self._transposed(G0, G1)
+        dp = torch.empty((B, G0, G1, C), dtype=torch.float32, device=dev)
+        fx = torch.empty(((G1 + 127) // 128, B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        gx = torch.empty((B * G0, C, 2 * self.mx), dtype=torch.float32, device=dev)
+        dO2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)
+        dF2 = torch.empty_like(dO2)
+        o.layer(0, B, G0, G1, None, None, CS=AAT, aux=dv, vout=dp, fx=fx)
+        dpre = dv  # the last layer has no GELU
+        for l in reversed(range(self.layers)):
+            o.csum(B, C, L, dpre, g[f"b{l + 1}"])
+            o.wgrad(C, C, L, dpre, c["v"][l], B, g[f"W{l + 1}"])
+            o.pdft(B, G0, G1, fx, DpivT, dO2)
+            o.mix(1, B, C, C, K, dO2, P[f"R{l}"], dF2)
+            o.mix(2, B, C, C, K, c["F2"][l], dO2, g[f"R{l}"])
+            o.pidft(B, G0, dF2, DpvT, gx)
+            dpre = torch.empty_like(dv)
+            o.layer(1, B, G0, G1, P[f"W{l + 1}"].t().contiguous(), None, act=2 if l > 0 else 0, vin=dp, gx=gx, AA=CST,
+                    CS=AAT, aux=c["pre"][l - 1] if l > 0 else None, vout=dp if l > 0 else None,
+                    fx=fx if l > 0 else None, vcm=dpre)
+        return dpre
 
     def _forward_fused(self, B, G0, G1, pr, xs_t, ps_t):
         """Inference: each layer reads and writes the activations once."""
@@ -322,6 +387,11 @@ class FNO2d:
         dv = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
         o.gemm(1, 0, C, L, PJ, P["Q1"], C, 0, da1, L, PJ * L, dv, L, C * L, B)
         del da1
+        if self._fused_layers(G0, G1):
+            dpre = self._layers_backward(dv, c)
+            o.csum(B, C, L, dpre, g["b0"])
+            o.wgrad(C, NP + 2, L, dpre, c["feats"], B, g["W0"])
+            return g
         dGx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev)
         dFx = torch.empty_like(dGx)
         dO2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)
