@@ -226,6 +226,184 @@ extern "C" int fw_fno_channel_sum(int Bn, int C, long long L, const float* X, fl
   return e == cudaSuccess ? FW_OK : cuda_fail(e, "fw_fno_channel_sum");
 }
 
+// ---------------------------------------------------------------------------
+// Weight gradients out[r][c] = sum_b sum_l dY[b][r][l] X[b][c][l] (and the bias
+// gradients sum dY[b][r][l]) over channel-major activations, in FP32 FMAs.  The
+// contraction runs over every pixel and gives 32 x 32 outputs a tile, so the
+// tensor core has nothing to reuse: its operands had to be split and stored to
+// shared memory for 12 MMAs a chunk (0.32 ms a layer at 16 x 256^2; this kernel
+// 0.07, near the time of reading both operands once).  A CTA stages 32 + 32 rows of
+// 128 pixels; each of its eight warps contracts 16 of them for the whole tile,
+// lane (rg, cg) owning rows rg + 8 i and columns cg + 4 j (128 FMAs per 12 vector
+// loads without bank conflicts).  A chain adds a few hundred pixels in FP32; warps
+// and CTAs are summed in FP64.
+namespace wgrad {
+constexpr int TP = 128, PITCH = TP + 4;
+constexpr size_t SMEM = (size_t)2 * 32 * PITCH * 4;
+}  // namespace wgrad
+
+__global__ void __launch_bounds__(256, 2) wgrad_kernel(int rows, int cols, long long L, long long range, int nr,
+                                                       const float* __restrict__ dY, long long sY,
+                                                       const float* __restrict__ X, long long sX, float* __restrict__ work,
+                                                       float* __restrict__ bwork) {
+  using namespace wgrad;
+  extern __shared__ __align__(16) float sm[];
+  float* Ys = sm;
+  float* Xs = sm + 32 * PITCH;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, cg = lane & 3;
+  const int r0 = (blockIdx.x % nr) * 32, c0 = (blockIdx.x / nr) * 32;
+  const int split = blockIdx.z * gridDim.y + blockIdx.y;  // (sample, range)
+  const long long l0 = (long long)blockIdx.y * range, l1 = l0 + range < L ? l0 + range : L;
+  const float* y = dY + (long long)blockIdx.z * sY;
+  const float* x = X + (long long)blockIdx.z * sX;
+  float acc[4][8], bs[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    bs[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  }
+  float4 ry[4], rx[4];
+  auto fetch = [&](long long l) {  // warp w: rows w, w + 8, ...; lane: four pixels
+    const bool in = l + 4 * lane < l1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + warp + 8 * i, c = c0 + warp + 8 * i;
+      ry[i] = in && r < rows ? __ldg(reinterpret_cast<const float4*>(y + r * L + l + 4 * lane)) : make_float4(0, 0, 0, 0);
+      rx[i] = in && c < cols ? __ldg(reinterpret_cast<const float4*>(x + c * L + l + 4 * lane)) : make_float4(0, 0, 0, 0);
+    }
+  };
+  fetch(l0);
+  for (long long l = l0; l < l1; l += TP) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(Ys + (warp + 8 * i) * PITCH + 4 * lane) = ry[i];
+      *reinterpret_cast<float4*>(Xs + (warp + 8 * i) * PITCH + 4 * lane) = rx[i];
+    }
+    __syncthreads();
+    if (l + TP < l1) fetch(l + TP);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int p = warp * 16 + 4 * q;
+      float4 b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(Xs + (cg + 4 * j) * PITCH + p);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(Ys + (rg + 8 * i) * PITCH + p);
+        bs[i] += (a.x + a.y) + (a.z + a.w);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
+          acc[i][j] = fmaf(a.y, b[j].y, acc[i][j]);
+          acc[i][j] = fmaf(a.z, b[j].z, acc[i][j]);
+          acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // the warps' tiles through shared memory (8 x 1024 floats), summed in FP64
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[warp * 1024 + (rg + 8 * i) * 32 + cg + 4 * j] = acc[i][j];
+  __syncthreads();
+  for (int e = tid; e < 1024; e += 256) {
+    const int r = r0 + (e >> 5), c = c0 + (e & 31);
+    double s = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += (double)sm[w * 1024 + e];
+    if (r < rows && c < cols) work[(long long)split * rows * cols + (long long)r * cols + c] = (float)s;
+  }
+  if (bwork != nullptr && c0 == 0) {
+    __syncthreads();
+    if (cg == 0)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sm[warp * 32 + rg + 8 * i] = bs[i];
+    __syncthreads();
+    if (tid < 32 && r0 + tid < rows) {
+      double s = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += (double)sm[w * 32 + tid];
+      bwork[(long long)split * rows + r0 + tid] = (float)s;
+    }
+  }
+}
+
+// out[e] = sum over Z slices (FP64) for the E weights, then the R bias sums
+__global__ void wgrad_sum_kernel(int Z, int E, int R, const float* __restrict__ work, const float* __restrict__ bwork,
+                                 float* out, float* bias) {
+  const int e = blockIdx.x * 32 + threadIdx.x;
+  const bool w = e < E;
+  double s = 0.0;
+  if (e < E + R)
+    for (int z = threadIdx.y; z < Z; z += 8) s += w ? (double)work[(long long)z * E + e] : (double)bwork[(long long)z * R + e - E];
+  __shared__ double red[8][33];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && e < E + R) {
+    double t = 0.0;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
+    if (w) out[e] = (float)t;
+    else bias[e - E] = (float)t;
+  }
+}
+
+// Pixel ranges per sample: two CTAs per SM over the launch, at least 512 pixels
+// a range (a multiple of the 128-pixel stage).
+static void wgrad_ranges(int rows, int cols, long long L, int batch, int* ns, long long* range) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long tiles = (long long)((rows + 31) / 32) * ((cols + 31) / 32) * batch;
+  long long want = (4LL * sms + tiles - 1) / tiles;
+  if (want > (L + 511) / 512) want = (L + 511) / 512;
+  if (want < 1) want = 1;
+  *range = ((L + want - 1) / want + wgrad::TP - 1) / wgrad::TP * wgrad::TP;
+  *ns = (int)((L + *range - 1) / *range);
+}
+
+static int wgrad_check(int rows, int cols, long long L, int batch) {
+  if (rows < 1 || cols < 1 || L < 4 || L % 4 != 0 || L > (1LL << 30) || batch < 1 || batch > 65535 || rows > 4096 || cols > 4096)
+    return fail(FW_EINVAL, "fw_fno_wgrad_bias: sizes must be positive, L a multiple of 4");
+  return FW_OK;
+}
+
+extern "C" int fw_fno_wgrad_bias_work(int rows, int cols, long long L, int batch, long long* floats_out) {
+  if (floats_out == nullptr) return fail(FW_EINVAL, "fw_fno_wgrad_bias_work: NULL argument");
+  if (int rc = wgrad_check(rows, cols, L, batch)) return rc;
+  int ns;
+  long long range;
+  wgrad_ranges(rows, cols, L, batch, &ns, &range);
+  *floats_out = (long long)batch * ns * rows * (cols + 1);
+  return FW_OK;
+}
+
+extern "C" int fw_fno_wgrad_bias(int rows, int cols, long long L, const float* dY, long long strideY, const float* X,
+                                 long long strideX, int batch, float* work, long long work_floats, float* out, float* bias,
+                                 void* stream) {
+  if (int rc = wgrad_check(rows, cols, L, batch)) return rc;
+  if (dY == nullptr || X == nullptr || work == nullptr || out == nullptr) return fail(FW_EINVAL, "fw_fno_wgrad_bias: NULL argument");
+  if ((((uintptr_t)dY | (uintptr_t)X) & 15u) != 0 || strideY % 4 != 0 || strideX % 4 != 0)
+    return fail(FW_EINVAL, "fw_fno_wgrad_bias: operands must start on 16 bytes");
+  int ns;
+  long long range;
+  wgrad_ranges(rows, cols, L, batch, &ns, &range);
+  const long long z = (long long)batch * ns;
+  if (work_floats < z * rows * (cols + 1)) return fail(FW_EINVAL, "fw_fno_wgrad_bias: work buffer too small");
+  float* bwork = bias != nullptr ? work + z * rows * cols : nullptr;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int nr = (rows + 31) / 32, nc = (cols + 31) / 32;
+  wgrad_kernel<<<dim3(nr * nc, ns, batch), 256, wgrad::SMEM, st>>>(rows, cols, L, range, nr, dY, strideY, X, strideX, work, bwork);
+  const int E = rows * cols, R = bias != nullptr ? rows : 0;
+  wgrad_sum_kernel<<<(E + R + 31) / 32, dim3(32, 8), 0, st>>>((int)z, E, R, work, bwork, out, bias);
+  count_launch(2);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? FW_OK : cuda_fail(e, "fw_fno_wgrad_bias");
+}
+
 extern "C" int fw_fno_rel_l2(int Bn, long long L, const float* Y, const float* T, float* dY, double* loss,
                              void* stream) {
   rel_l2_kernel<<<Bn, 256, 0, static_cast<cudaStream_t>(stream)>>>(L, Y, T, dY, loss, Bn);

@@ -68,6 +68,18 @@ class _Ops:
         check(self.lib.fw_fno_wgrad(rows, cols, L, _p(dY), rows * L, _p(X), cols * L, batch, _p(self._work),
                                     self._work.numel(), _p(out), 0, stream_handle()), "fw_fno_wgrad")
 
+    def wgrad_bias(self, rows, cols, L, dY, X, batch, out, bias):
+        """wgrad and csum in one pass: out, and bias[r] = sum_b sum_l dY[b][r][l]."""
+        if L % 4:  # (rows off 16 bytes)
+            self.csum(batch, rows, L, dY, bias)
+            return self.wgrad(rows, cols, L, dY, X, batch, out)
+        n = ctypes.c_longlong(0)
+        check(self.lib.fw_fno_wgrad_bias_work(rows, cols, L, batch, ctypes.byref(n)), "fw_fno_wgrad_bias_work")
+        if self._work is None or self._work.numel() < n.value:
+            self._work = torch.empty(n.value, dtype=torch.float32, device=dY.device)
+        check(self.lib.fw_fno_wgrad_bias(rows, cols, L, _p(dY), rows * L, _p(X), cols * L, batch, _p(self._work),
+                                         self._work.numel(), _p(out), _p(bias), stream_handle()), "fw_fno_wgrad_bias")
+
     def project(self, hidden, C, L, V, batch, Q1, c1, Q2, c2, out):
         check(self.lib.fw_fno_project(hidden, C, L, _p(V), C * L, batch, _p(Q1), _p(c1), _p(Q2), _p(c2), _p(out), L,
                                       stream_handle()), "fw_fno_project")
@@ -331,8 +343,7 @@ class FNO2d:
         o.layer(0, B, G0, G1, None, None, CS=AAT, aux=dv, vout=dp, fx=fx)
         dpre = dv  # the last layer has no GELU
         for l in reversed(range(self.layers)):
-            o.csum(B, C, L, dpre, g[f"b{l + 1}"])
-            o.wgrad(C, C, L, dpre, c["v"][l], B, g[f"W{l + 1}"])
+            o.wgrad_bias(C, C, L, dpre, c["v"][l], B, g[f"W{l + 1}"], g[f"b{l + 1}"])
             o.pdft(B, G0, G1, fx, DpivT, dO2)
             o.mix(1, B, C, C, K, dO2, P[f"R{l}"], dF2)
             o.mix(2, B, C, C, K, c["F2"][l], dO2, g[f"R{l}"])
@@ -377,20 +388,17 @@ class FNO2d:
         CS, Dpv, Dpiv, AA = self._grid(G0, G1)
         dev = self.device
         d_out = dout.contiguous().view(B, 1, G0, G1)
-        o.csum(B, 1, L, d_out, g["c2"])
-        o.wgrad(1, PJ, L, d_out, c["a1"], B, g["Q2"])
+        o.wgrad_bias(1, PJ, L, d_out, c["a1"], B, g["Q2"], g["c2"])
         # da1 = GELU'(pre1) Q2^T d_out
         da1 = torch.empty((B, PJ, G0, G1), dtype=torch.float32, device=dev)
         o.gemm_ex(1, 0, PJ, L, 1, P["Q2"], PJ, 0, d_out, L, L, da1, L, PJ * L, B, aux=c["pre1"], act=2)
-        o.csum(B, PJ, L, da1, g["c1"])
-        o.wgrad(PJ, C, L, da1, c["vL"], B, g["Q1"])
+        o.wgrad_bias(PJ, C, L, da1, c["vL"], B, g["Q1"], g["c1"])
         dv = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
         o.gemm(1, 0, C, L, PJ, P["Q1"], C, 0, da1, L, PJ * L, dv, L, C * L, B)
         del da1
         if self._fused_layers(G0, G1):
             dpre = self._layers_backward(dv, c)
-            o.csum(B, C, L, dpre, g["b0"])
-            o.wgrad(C, NP + 2, L, dpre, c["feats"], B, g["W0"])
+            o.wgrad_bias(C, NP + 2, L, dpre, c["feats"], B, g["W0"], g["b0"])
             return g
         dGx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev)
         dFx = torch.empty_like(dGx)
@@ -398,9 +406,7 @@ class FNO2d:
         dF2 = torch.empty_like(dO2)
         dpre = dv  # the last layer has no GELU
         for l in reversed(range(self.layers)):
-            o.csum(B, C, L, dpre, g[f"b{l + 1}"])
-            vin = c["v"][l]
-            o.wgrad(C, C, L, dpre, vin, B, g[f"W{l + 1}"])
+            o.wgrad_bias(C, C, L, dpre, c["v"][l], B, g[f"W{l + 1}"], g[f"b{l + 1}"])
             dvin = torch.empty_like(dpre)
             o.gemm(1, 0, C, L, C, P[f"W{l + 1}"], C, 0, dpre, L, C * L, dvin, L, C * L, B)
             # spectral path
@@ -417,8 +423,7 @@ class FNO2d:
             else:
                 o.gemm(0, 1, G0, G1, 2 * mx, dFx, 2 * mx, 2 * G0 * mx, CS, 2 * mx, 0, dvin, G1, L, B * C, beta=1.0)
             dpre = dvin
-        o.csum(B, C, L, dpre, g["b0"])
-        o.wgrad(C, NP + 2, L, dpre, c["feats"], B, g["W0"])
+        o.wgrad_bias(C, NP + 2, L, dpre, c["feats"], B, g["W0"], g["b0"])
         return g
 
     def adam_step(self, lr, wd=0.0):

@@ -363,6 +363,12 @@ int fw_fno_wgrad_work(int rows, int cols, long long L, int batch, long long* flo
 int fw_fno_wgrad(int rows, int cols, long long L, const float* dY, long long strideY, const float* X,
                  long long strideX, int batch, float* work, long long work_floats, float* out, int accumulate,
                  void* stream);
+/* The same weight gradient and, with bias != NULL, bias[r] = sum_b sum_l dY[b][r][l], in FP32 FMAs with FP64 sums of
+ * the slices; L and the strides multiples of 4, operands on 16 bytes; work: fw_fno_wgrad_bias_work floats. */
+int fw_fno_wgrad_bias_work(int rows, int cols, long long L, int batch, long long* floats_out);
+int fw_fno_wgrad_bias(int rows, int cols, long long L, const float* dY, long long strideY, const float* X,
+                      long long strideX, int batch, float* work, long long work_floats, float* out, float* bias,
+                      void* stream);
 /* Fused two-layer pointwise projection: out[b][l] = c2[0] + sum_j Q2[j] GELU(c1[j] +
  * sum_c Q1[j][c] V[b][c][l]) for j < hidden <= 128 (Q1: hidden x C); the hidden layer
  * stays in tensor memory. */

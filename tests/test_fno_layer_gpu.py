@@ -77,3 +77,21 @@ def test_fused_forward_matches_unfused(G0, G1):
     assert net._fused_layers(G0, G1)
     a, b = net.forward(X, xs, ps, cache=False), net.forward(X, xs, ps, cache=True)
     assert (a - b).abs().max() <= 2e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("rows,cols,L,B", [(32, 32, 65536, 2), (1, 128, 4100, 3), (128, 32, 1028, 1), (32, 5, 132, 4),
+                                           (33, 40, 4, 2)])
+def test_weight_and_bias_gradients(rows, cols, L, B):
+    """fw_fno_wgrad_bias: tiles of 32 x 32 with ragged edges, pixel ranges that end
+    inside a 128-pixel stage, one to many ranges per sample."""
+    from fastwigner_b200.fno import _Ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    dY = torch.randn(B, rows, L, device="cuda", generator=g)
+    X = torch.randn(B, cols, L, device="cuda", generator=g)
+    out, bias = torch.full((rows, cols), float("nan"), device="cuda"), torch.full((rows,), float("nan"), device="cuda")
+    _Ops().wgrad_bias(rows, cols, L, dY, X, B, out, bias)
+    # sums of B L products of unit variance: FP32 chains of a few hundred terms, FP64 above
+    tol = 1e-6 * (B * L) ** 0.5 * 10
+    assert (out.double() - torch.einsum("brl,bcl->rc", dY.double(), X.double())).abs().max() < tol
+    assert (bias.double() - dY.double().sum(dim=(0, 2))).abs().max() < tol
