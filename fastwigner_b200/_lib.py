@@ -99,6 +99,8 @@ _SIGNATURES = [
     ("fw_fno_wgrad", c_int, [c_int, c_int, c_ll, c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_int, c_vp]),
     ("fw_fno_wgrad_bias_work", c_int, [c_int, c_int, c_ll, c_int, ctypes.POINTER(c_ll)]),
     ("fw_fno_wgrad_bias", c_int, [c_int, c_int, c_ll, c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_vp, c_vp]),
+    ("fw_fno_project_bwd_work", c_int, [c_ll, c_int, ctypes.POINTER(c_ll)]),
+    ("fw_fno_project_bwd", c_int, [c_ll, c_int, c_vp, c_ll] + [c_vp] * 6 + [c_ll] + [c_vp] * 5),
     ("fw_fno_project", c_int, [c_int, c_int, c_ll, c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp]),
     ("fw_fno_layer", c_int, [c_int] * 4 + [c_vp] * 6 + [c_int] * 2 + [c_vp] * 14),
     ("fw_fno_pdft", c_int, [c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),

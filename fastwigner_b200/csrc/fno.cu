@@ -404,6 +404,264 @@ extern "C" int fw_fno_wgrad_bias(int rows, int cols, long long L, const float* d
   return e == cudaSuccess ? FW_OK : cuda_fail(e, "fw_fno_wgrad_bias");
 }
 
+// ---------------------------------------------------------------------------
+// Backward pass of the projection out = Q2 GELU(Q1 v + c1) + c2 (128 hidden, 32
+// channels) for d = d(loss)/d(out): the hidden layer is evaluated again tile by
+// tile, so neither it nor its gradient touches memory (128 channels of 4 bytes a
+// pixel, written twice and read five times as separate products: 2.9 ms at
+// 16 x 256^2; this kernel reads v and d and writes dv).  Per tile of 64 pixels:
+//   h = Q1 v + c1;  dh = Q2 d GELU'(h);  dc1 += dh;  dQ2 += GELU(h) d     4 x 8 (j, x) a thread
+//   dv = Q1^T dh                                   4 x 8 (c, x) a thread, a quarter of j each
+//   dQ1 += dh v^T                                  4 x 4 (j, c) a thread
+// Every product reads two or three 16-byte vectors per 32 FMAs.  Tile sums add up
+// in FP64.
+namespace projb {
+constexpr int H = 128, C = 32, TX = 64, PX = TX + 4;
+constexpr int F_Q1T = 0, F_Q1N = C * H, F_V = 2 * C * H, F_D = F_V + C * PX, F_DH = F_D + TX, F_RED = F_DH + H * PX,
+              FLOATS = F_RED + 4 * C * PX;
+constexpr int REC = H * C + 2 * H + 1;  // dQ1, dc1, dQ2, dc2 of a block
+}  // namespace projb
+
+__global__ void __launch_bounds__(256, 2) project_bwd_kernel(long long L, int batch, const float* __restrict__ V, long long sV,
+                                                             const float* __restrict__ Q1, const float* __restrict__ c1,
+                                                             const float* __restrict__ Q2, const float* __restrict__ dout,
+                                                             float* __restrict__ dV, double* __restrict__ work) {
+  using namespace projb;
+  extern __shared__ __align__(16) float sm[];
+  float *q1t = sm + F_Q1T, *q1n = sm + F_Q1N, *vs = sm + F_V, *ds = sm + F_D, *dh = sm + F_DH, *red = sm + F_RED;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < H * C; i += 256) {
+    const float q = __ldg(Q1 + i);
+    q1n[i] = q;
+    q1t[(i % C) * H + i / C] = q;
+  }
+  const int tj = tid >> 3, t8 = tid & 7;  // hidden rows 4 tj .. + 3 (h), tj + 32 i (dQ1); pixels 4 t8, 32 + 4 t8; channels t8 + 8 i
+  float b1[4], w2[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    b1[i] = __ldg(c1 + 4 * tj + i);
+    w2[i] = __ldg(Q2 + 4 * tj + i);
+  }
+  double gq[4][4], gc[4], g2[4], gd = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    gc[i] = g2[i] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gq[i][j] = 0;
+  }
+  const long long per = (L + TX - 1) / TX, total = per * batch;
+  const long long first = blockIdx.x * total / gridDim.x, last = (blockIdx.x + 1) * total / gridDim.x;
+  float4 rv[2], rd;
+  auto fetch = [&](long long t) {
+    const long long b = t / per, l = (t - b * per) * TX;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = (tid >> 4) + 16 * i;
+      const long long p = l + 4 * (tid & 15);
+      rv[i] = p < L ? __ldg(reinterpret_cast<const float4*>(V + b * sV + c * L + p)) : make_float4(0, 0, 0, 0);
+    }
+    if (tid < TX / 4) {
+      const long long p = l + 4 * tid;
+      rd = p < L ? __ldg(reinterpret_cast<const float4*>(dout + b * L + p)) : make_float4(0, 0, 0, 0);
+    }
+  };
+  if (first < last) fetch(first);
+  for (long long t = first; t < last; ++t) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(vs + ((tid >> 4) + 16 * i) * PX + 4 * (tid & 15)) = rv[i];
+    if (tid < TX / 4) {
+      *reinterpret_cast<float4*>(ds + 4 * tid) = rd;
+      gd += ((double)rd.x + (double)rd.y) + ((double)rd.z + (double)rd.w);
+    }
+    __syncthreads();
+    if (t + 1 < last) fetch(t + 1);
+    auto put = [](float (&f)[8], const float4 a, const float4 b) {
+      f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+    };
+    auto row8 = [&](float (&f)[8], const float* r) {
+      put(f, *reinterpret_cast<const float4*>(r + 4 * t8), *reinterpret_cast<const float4*>(r + 32 + 4 * t8));
+    };
+    {  // hidden layer and its gradient
+      float h[4][8], x[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) h[i][k] = 0.f;
+#pragma unroll 8
+      for (int c = 0; c < C; ++c) {
+        const float4 q = *reinterpret_cast<const float4*>(q1t + c * H + 4 * tj);
+        row8(x, vs + c * PX);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          h[0][k] = fmaf(q.x, x[k], h[0][k]);
+          h[1][k] = fmaf(q.y, x[k], h[1][k]);
+          h[2][k] = fmaf(q.z, x[k], h[2][k]);
+          h[3][k] = fmaf(q.w, x[k], h[3][k]);
+        }
+      }
+      row8(x, ds);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float sc = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float u = h[i][k] + b1[i];
+          s2 = fmaf(gelu(u), x[k], s2);
+          h[i][k] = w2[i] * x[k] * gelu_d(u);
+          sc += h[i][k];
+        }
+        gc[i] += (double)sc;
+        g2[i] += (double)s2;
+        float* r = dh + (4 * tj + i) * PX;
+        *reinterpret_cast<float4*>(r + 4 * t8) = make_float4(h[i][0], h[i][1], h[i][2], h[i][3]);
+        *reinterpret_cast<float4*>(r + 32 + 4 * t8) = make_float4(h[i][4], h[i][5], h[i][6], h[i][7]);
+      }
+    }
+    __syncthreads();
+    {  // input gradient, hidden rows 32 jg .. + 31
+      const int jg = tid >> 6, tc = (tid >> 3) & 7;
+      float g[4][8], x[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) g[i][k] = 0.f;
+#pragma unroll 8
+      for (int jj = 0; jj < 32; ++jj) {
+        const int j = 32 * jg + jj;
+        const float4 q = *reinterpret_cast<const float4*>(q1n + j * C + 4 * tc);
+        row8(x, dh + j * PX);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          g[0][k] = fmaf(q.x, x[k], g[0][k]);
+          g[1][k] = fmaf(q.y, x[k], g[1][k]);
+          g[2][k] = fmaf(q.z, x[k], g[2][k]);
+          g[3][k] = fmaf(q.w, x[k], g[3][k]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float* r = red + (jg * C + 4 * tc + i) * PX;
+        *reinterpret_cast<float4*>(r + 4 * t8) = make_float4(g[i][0], g[i][1], g[i][2], g[i][3]);
+        *reinterpret_cast<float4*>(r + 32 + 4 * t8) = make_float4(g[i][4], g[i][5], g[i][6], g[i][7]);
+      }
+    }
+    {  // weight gradient
+      float w[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[i][j] = 0.f;
+#pragma unroll 4
+      for (int p = 0; p < TX; p += 4) {
+        float4 b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(vs + (t8 + 8 * j) * PX + p);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 q = *reinterpret_cast<const float4*>(dh + (tj + 32 * i) * PX + p);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) w[i][j] = fmaf(q.w, b[j].w, fmaf(q.z, b[j].z, fmaf(q.y, b[j].y, fmaf(q.x, b[j].x, w[i][j]))));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gq[i][j] += (double)w[i][j];
+    }
+    __syncthreads();
+    const long long b = t / per, l = (t - b * per) * TX;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = (tid >> 4) + 16 * i, x = 4 * (tid & 15);
+      float4 s = *reinterpret_cast<const float4*>(red + c * PX + x);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        const float4 u = *reinterpret_cast<const float4*>(red + (k * C + c) * PX + x);
+        s.x += u.x, s.y += u.y, s.z += u.z, s.w += u.w;
+      }
+      if (l + x < L) *reinterpret_cast<float4*>(dV + (b * C + c) * L + l + x) = s;
+    }
+  }
+  // the block's sums; gc, g2 over the eight threads that share hidden rows, gd over the loaders
+  double* rec = work + (long long)blockIdx.x * REC;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) rec[(tj + 32 * i) * C + t8 + 8 * j] = gq[i][j];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      gc[i] += __shfl_xor_sync(0xffffffffu, gc[i], o);
+      g2[i] += __shfl_xor_sync(0xffffffffu, g2[i], o);
+    }
+    if (t8 == 0) {
+      rec[H * C + 4 * tj + i] = gc[i];
+      rec[H * C + H + 4 * tj + i] = g2[i];
+    }
+  }
+  if (tid < 32) {
+    for (int o = 16; o > 0; o >>= 1) gd += __shfl_xor_sync(0xffffffffu, gd, o);
+    if (tid == 0) rec[REC - 1] = gd;
+  }
+}
+
+__global__ void project_bwd_sum_kernel(int blocks, const double* __restrict__ work, float* gQ1, float* gc1, float* gQ2, float* gc2) {
+  using namespace projb;
+  const int e = blockIdx.x * 32 + threadIdx.x;
+  double s = 0.0;
+  if (e < REC)
+    for (int z = threadIdx.y; z < blocks; z += 8) s += work[(long long)z * REC + e];
+  __shared__ double red[8][33];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0 || e >= REC) return;
+  double t = 0.0;
+#pragma unroll
+  for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
+  if (e < H * C) gQ1[e] = (float)t;
+  else if (e < H * C + H) gc1[e - H * C] = (float)t;
+  else if (e < REC - 1) gQ2[e - H * C - H] = (float)t;
+  else gc2[0] = (float)t;
+}
+
+static int project_bwd_blocks(long long L, int batch) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long tiles = (L + projb::TX - 1) / projb::TX * batch;
+  return (int)(tiles < 2LL * sms ? tiles : 2LL * sms);
+}
+
+extern "C" int fw_fno_project_bwd_work(long long L, int batch, long long* doubles_out) {
+  if (doubles_out == nullptr || L < 4 || L % 4 != 0 || L > (1LL << 30) || batch < 1 || batch > 65535)
+    return fail(FW_EINVAL, "fw_fno_project_bwd_work: bad argument");
+  *doubles_out = (long long)project_bwd_blocks(L, batch) * projb::REC;
+  return FW_OK;
+}
+
+extern "C" int fw_fno_project_bwd(long long L, int batch, const float* V, long long strideV, const float* Q1, const float* c1,
+                                  const float* Q2, const float* dout, float* dV, double* work, long long work_doubles,
+                                  float* gQ1, float* gc1, float* gQ2, float* gc2, void* stream) {
+  long long need = 0;
+  if (int rc = fw_fno_project_bwd_work(L, batch, &need)) return rc;
+  if (V == nullptr || Q1 == nullptr || c1 == nullptr || Q2 == nullptr || dout == nullptr || dV == nullptr || work == nullptr ||
+      gQ1 == nullptr || gc1 == nullptr || gQ2 == nullptr || gc2 == nullptr)
+    return fail(FW_EINVAL, "fw_fno_project_bwd: NULL argument");
+  if ((((uintptr_t)V | (uintptr_t)dout | (uintptr_t)dV) & 15u) != 0 || strideV % 4 != 0)
+    return fail(FW_EINVAL, "fw_fno_project_bwd: activations must start on 16 bytes");
+  if (work_doubles < need) return fail(FW_EINVAL, "fw_fno_project_bwd: work buffer too small");
+  constexpr size_t smem = (size_t)projb::FLOATS * 4;
+  static PerDeviceOnce attr;
+  cudaError_t e = set_smem_once(attr, project_bwd_kernel, smem);
+  if (e != cudaSuccess) return cuda_fail(e, "fw_fno_project_bwd");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int blocks = project_bwd_blocks(L, batch);
+  project_bwd_kernel<<<blocks, 256, smem, st>>>(L, batch, V, strideV, Q1, c1, Q2, dout, dV, work);
+  project_bwd_sum_kernel<<<(projb::REC + 31) / 32, dim3(32, 8), 0, st>>>(blocks, work, gQ1, gc1, gQ2, gc2);
+  count_launch(2);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? FW_OK : cuda_fail(e, "fw_fno_project_bwd");
+}
+
 extern "C" int fw_fno_rel_l2(int Bn, long long L, const float* Y, const float* T, float* dY, double* loss,
                              void* stream) {
   rel_l2_kernel<<<Bn, 256, 0, static_cast<cudaStream_t>(stream)>>>(L, Y, T, dY, loss, Bn);

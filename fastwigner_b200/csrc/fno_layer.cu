@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
 #pragma unroll
       for (int i = 0; i < LC; ++i) v[i] = 0.f;
     }
-    if (MODE != LAYER_LAST && a.vcm != nullptr && st < nx) {
+    if (a.vcm != nullptr && st < nx) {
       float* p = a.vcm + cm_base(r);
 #pragma unroll
       for (int i = 0; i < LC; ++i) p[i * chs] = v[i];

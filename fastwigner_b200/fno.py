@@ -107,6 +107,14 @@ class _Ops:
     def pidft(self, B, G0, O2, Dpiv, gx):
         check(self.lib.fw_fno_pidft(B, G0, _p(O2), _p(Dpiv), _p(gx), stream_handle()), "fw_fno_pidft")
 
+    def project_bwd(self, L, B, V, Q1, c1, Q2, dout, dV, gQ1, gc1, gQ2, gc2):
+        n = ctypes.c_longlong(0)
+        check(self.lib.fw_fno_project_bwd_work(L, B, ctypes.byref(n)), "fw_fno_project_bwd_work")
+        work = torch.empty(n.value, dtype=torch.float64, device=V.device)
+        check(self.lib.fw_fno_project_bwd(L, B, _p(V), V[0].numel(), _p(Q1), _p(c1), _p(Q2), _p(dout), _p(dV),
+                                          ctypes.c_void_p(work.data_ptr()), n.value, _p(gQ1), _p(gc1), _p(gQ2), _p(gc2),
+                                          stream_handle()), "fw_fno_project_bwd")
+
     def mix(self, mode, B, Ci, Co, K, X, Y, out):
         check(self.lib.fw_fno_mix(mode, B, Ci, Co, K, _p(X), _p(Y), _p(out), stream_handle()), "fw_fno_mix")
 
@@ -245,12 +253,14 @@ class FNO2d:
         if not self._fused_layers(G0, G1):
             o.gemm_ex(0, 0, C, L, NP + 2, P["W0"], NP + 2, 0, feats, L, (NP + 2) * L, v, L, C * L, B, bias=P["b0"])
         Kp, mx, K = self.Kp, self.mx, self.K
-        fused = self._fused_layers(G0, G1)
-        if fused:
-            v = self._layers_cached(c, v, CS, Dpv, Dpiv, AA)
-        Fx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev) if not fused else None
-        Gx = torch.empty_like(Fx) if not fused else None
-        for l in range(0 if fused else self.layers):
+        if self._fused_layers(G0, G1):
+            out = torch.empty((B, G0, G1), dtype=torch.float32, device=dev)
+            c["vL"] = self._layers_cached(c, v, CS, Dpv, Dpiv, AA, out)
+            self._cache = c
+            return out
+        Fx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev)
+        Gx = torch.empty_like(Fx)
+        for l in range(self.layers):
             if cache:
                 c["v"].append(v)
             # truncated forward DFT: x (cosine and sine parts in one product), then p
@@ -294,9 +304,10 @@ class FNO2d:
         return (self.C == 32 and self.mp == self.mx == 16 and self.proj == 128 and self.layers >= 1
                 and self.NP <= 14 and 32 <= G0 <= 1024 and G1 >= 32 and G1 % 4 == 0)
 
-    def _layers_cached(self, c, v, CS, Dpv, Dpiv, AA):
-        """The lift (into v) and the layers by the fused kernels, keeping for the
-        backward pass what the unfused ones keep; returns the last layer's output."""
+    def _layers_cached(self, c, v, CS, Dpv, Dpiv, AA, out):
+        """The lift (into v), the layers and the projection (into out) by the fused
+        kernels, keeping for the backward pass what the unfused ones keep except
+        the projection's hidden layer; returns the last layer's output."""
         o, P, dev, C, K = self.ops, self.params, self.device, self.C, self.K
         B, G0, G1 = c["B"], c["G0"], c["G1"]
         pr, xs_t, ps_t = c["lift"]
@@ -313,11 +324,14 @@ class FNO2d:
             o.mix(0, B, C, C, K, F2, P[f"R{l}"], O2)
             o.pidft(B, G0, O2, Dpiv, gx)
             v = torch.empty_like(v)
-            last = l == self.layers - 1
-            pre = None if last else torch.empty_like(v)
-            o.layer(1, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], act=int(not last), vin=vp, gx=gx, AA=AA, CS=CS,
-                    vout=None if last else vp, fx=None if last else fx, pre=pre, vcm=v)
-            c["pre"].append(pre)
+            if l < self.layers - 1:
+                pre = torch.empty_like(v)
+                o.layer(1, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], act=1, vin=vp, gx=gx, AA=AA, CS=CS, vout=vp,
+                        fx=fx, pre=pre, vcm=v)
+                c["pre"].append(pre)
+            else:
+                o.layer(2, B, G0, G1, P[f"W{l + 1}"], P[f"b{l + 1}"], vin=vp, gx=gx, AA=AA, Q1=P["Q1"], c1=P["c1"],
+                        Q2=P["Q2"], c2=P["c2"], out=out, vcm=v)
         return v
 
     def _transposed(self, G0, G1):
@@ -388,6 +402,12 @@ class FNO2d:
         CS, Dpv, Dpiv, AA = self._grid(G0, G1)
         dev = self.device
         d_out = dout.contiguous().view(B, 1, G0, G1)
+        if self._fused_layers(G0, G1):
+            dv = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
+            o.project_bwd(L, B, c["vL"], P["Q1"], P["c1"], P["Q2"], d_out, dv, g["Q1"], g["c1"], g["Q2"], g["c2"])
+            dpre = self._layers_backward(dv, c)
+            o.wgrad_bias(C, NP + 2, L, dpre, c["feats"], B, g["W0"], g["b0"])
+            return g
         o.wgrad_bias(1, PJ, L, d_out, c["a1"], B, g["Q2"], g["c2"])
         # da1 = GELU'(pre1) Q2^T d_out
         da1 = torch.empty((B, PJ, G0, G1), dtype=torch.float32, device=dev)
@@ -396,10 +416,6 @@ class FNO2d:
         dv = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
         o.gemm(1, 0, C, L, PJ, P["Q1"], C, 0, da1, L, PJ * L, dv, L, C * L, B)
         del da1
-        if self._fused_layers(G0, G1):
-            dpre = self._layers_backward(dv, c)
-            o.wgrad_bias(C, NP + 2, L, dpre, c["feats"], B, g["W0"], g["b0"])
-            return g
         dGx = torch.empty((B * C, G0, 2 * mx), dtype=torch.float32, device=dev)
         dFx = torch.empty_like(dGx)
         dO2 = torch.empty((B, C, 2, K), dtype=torch.float32, device=dev)

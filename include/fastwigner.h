@@ -380,7 +380,7 @@ int fw_fno_project(int hidden, int C, long long L, const float* V, long long str
  * mode 2: the same, then out = Q2 GELU(Q1 v' + c1) + c2 (128 hidden) and nothing else.  Modes 0 and 1 also write fx, the
  * forward x-transform of v' (CS: G1 x 32) per 128-pixel tile: [ceil(G1/128)][B G0][32 channels][32 parts]; with fx (and
  * vout) NULL only the channel-major copies.  Channel-major arrays, [B][32][G0][G1], for training: vcm (v'), pre (the
- * pre-activation, mode 1); aux: act 2 multiplies by GELU'(aux) (a layer's backward: CS^T and AA^T for AA and CS, W^T for
+ * pre-activation, mode 1; vcm in mode 2 too); aux: act 2 multiplies by GELU'(aux) (a layer's backward: CS^T and AA^T for AA and CS, W^T for
  * W), and mode 0 with aux copies it instead of lifting.
  * G0 in [32, 1024], G1 >= 32 a multiple of 4, NP <= 14. */
 int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float* gx, const float* AA, const float* CS,
@@ -395,6 +395,13 @@ int fw_fno_pidft(int B, int G0, const float* O2, const float* Dpiv, float* gx, v
  * harmonic state exp(-c H), H = p^2/2 + w^2 (x - x_e)^2/2, of unit sum; wc: (w, c) per sample; work: 64 B doubles. */
 int fw_fno_thermal(int B, int G0, int G1, const double* wc, const double* xs, const double* ps, double x_e, double dxdp,
                    float* out, double* work, void* stream);
+/* Backward of the projection (128 hidden, 32 channels) for dout = d(loss)/d(out): dV[b][32][L] and the gradients of Q1,
+ * c1, Q2, c2, the hidden layer evaluated again; L and strideV multiples of 4, activations on 16 bytes; work:
+ * fw_fno_project_bwd_work doubles. */
+int fw_fno_project_bwd_work(long long L, int batch, long long* doubles_out);
+int fw_fno_project_bwd(long long L, int batch, const float* V, long long strideV, const float* Q1, const float* c1,
+                       const float* Q2, const float* dout, float* dV, double* work, long long work_doubles, float* gQ1,
+                       float* gc1, float* gQ2, float* gc2, void* stream);
 /* Synchronous read of the FNO status word (0 or FW_FNO_TIMEOUT); clear != 0 resets it. */
 int fw_fno_status(int* status_out, int clear);
 /* Per-mode complex channel mixing, [B][C][2][K] layouts (real block, imaginary block):

@@ -95,3 +95,40 @@ def test_weight_and_bias_gradients(rows, cols, L, B):
     tol = 1e-6 * (B * L) ** 0.5 * 10
     assert (out.double() - torch.einsum("brl,bcl->rc", dY.double(), X.double())).abs().max() < tol
     assert (bias.double() - dY.double().sum(dim=(0, 2))).abs().max() < tol
+
+
+@pytest.mark.parametrize("G0,G1,B", [(32, 36, 1), (48, 192, 2), (64, 132, 3)])
+def test_training_gradients_match_autograd(G0, G1, B):
+    """One loss_and_grad + backward on the fused path (layers both ways, projection
+    backward, weight gradients) against FP64 autograd, 2e-5 of each gradient's
+    maximum (a gradient is a chain of about ten products of 1e-6 each)."""
+    from fastwigner_b200.fno import FNO2d
+
+    net = FNO2d(seed=2)
+    assert net._fused_layers(G0, G1)
+    rng = np.random.default_rng(7)
+    X = rng.uniform(0, 1, (B, 3))
+    xs, ps = np.linspace(-1, 1, G1, endpoint=False), np.linspace(-1, 1, G0, endpoint=False)
+    T = torch.tensor(rng.normal(size=(B, G0, G1)), dtype=torch.float32, device="cuda")
+    loss, dY = net.loss_and_grad(X, xs, ps, T)
+    grads = net.backward(dY)
+    p = {k: v.double().detach().requires_grad_() for k, v in net.params.items()}
+    f32 = lambda a: torch.tensor(np.asarray(a), dtype=torch.float32, device="cuda").double()  # noqa: E731
+    feats = torch.cat([f32(X)[:, :, None, None].expand(B, 3, G0, G1), f32(xs)[None, None, None, :].expand(B, 1, G0, G1),
+                       f32(ps)[None, None, :, None].expand(B, 1, G0, G1)], dim=1)
+    ch = lambda W, b, u: torch.einsum("oi,bixy->boxy", W, u) + b[None, :, None, None]  # noqa: E731
+    kp = np.concatenate([np.arange(16), np.arange(G0 - 16, G0)])
+    v = ch(p["W0"], p["b0"], feats)
+    for l in range(4):
+        F = torch.fft.rfft2(v, norm="forward")[:, :, kp, :16].reshape(B, 32, 512)
+        O = torch.einsum("bik,iok->bok", F, torch.complex(p[f"R{l}"][:, :, 0], p[f"R{l}"][:, :, 1])).reshape(B, 32, 32, 16)
+        full = torch.zeros((B, 32, G0, G1 // 2 + 1), dtype=O.dtype, device="cuda")
+        full[:, :, kp, :16] = O
+        y = torch.fft.irfft(torch.fft.ifft(full, dim=2, norm="forward"), n=G1, dim=3, norm="forward")
+        v = y + ch(p[f"W{l + 1}"], p[f"b{l + 1}"], v)
+        if l < 3:
+            v = torch.nn.functional.gelu(v)
+    Y = ch(p["Q2"], p["c2"], torch.nn.functional.gelu(ch(p["Q1"], p["c1"], v)))[:, 0]
+    ((Y - T.double()) ** 2).sum(dim=(1, 2)).div((T.double() ** 2).sum(dim=(1, 2))).mean().backward()
+    for k, t in p.items():
+        close(grads[k], t.grad, 2e-5)
