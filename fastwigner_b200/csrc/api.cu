@@ -53,7 +53,7 @@ static std::vector<double> stage_twiddles(int n, int rv) {
   return t;
 }
 
-static int upload_twiddles(int n, int dtype, void** dev, int rv = 0) {
+int upload_twiddles(int n, int dtype, void** dev, int rv) {
   std::vector<double> t = rv > 0 ? stage_twiddles(n, rv) : twiddles(n);
   cudaError_t e;
   if (dtype == FW_F64) {
@@ -109,8 +109,8 @@ extern "C" int fw_wigner_plan_create(int P, int X, int batch, int dtype, fw_wign
   if (np <= 0) return fail(FW_EINVAL, "fw_wigner_plan_create: unsupported X for the column pass tile");
   fw_wigner_plan* p = new fw_wigner_plan();
   p->P = P; p->X = X; p->batch = batch; p->dtype = dtype; p->nparts = np; p->small = small;
-  int rc = upload_twiddles(P, dtype, &p->twP);
-  if (rc == FW_OK) rc = upload_twiddles(X, dtype, &p->twX);
+  int rc = upload_twiddles(P, dtype, &p->twP, 0);
+  if (rc == FW_OK) rc = upload_twiddles(X, dtype, &p->twX, 0);
   if (rc == FW_OK) rc = upload_twiddles(X, dtype, &p->twsX, row_rv(dtype, X, small));
   if (rc == FW_OK) {
     cudaError_t e = cudaMalloc(&p->ring, sizeof(double) * 2 * (size_t)batch * np * MMAX);

@@ -226,28 +226,7 @@ template <typename Rl, int T> struct GroupEx {
 };
 
 // Exchange for the column passes: CP independent FFTs (one per column pair)
-// interleaved element-wise in one CTA-wide SoA buffer: element i of FFT c at
-// row-slot (i ^ ((i >> S) & 1)) * CP + c.  The xor of bit 0 with bit S puts the
-// two FFT indices that share a warp in different bank halves for both the
-// Stockham write and read patterns.  Synchronisation is CTA-wide.
-template <typename Rl, int CP, int S> struct ColEx {
-  Rl* re;
-  Rl* im;
-  int c;
-  using C = cplx_t<Rl>;
-  static constexpr int kL = 0;
-  static constexpr bool kFold = false;
-  __device__ __forceinline__ int map(int i) const { return (i ^ ((i >> S) & 1)) * CP + c; }
-  __device__ __forceinline__ static constexpr int delta(int) { return 0; }
-  __device__ __forceinline__ C read_at(int a) const { return mk<C>(re[a], im[a]); }
-  __device__ __forceinline__ void write_at(int a, C v) const { re[a] = v.x; im[a] = v.y; }
-  __device__ __forceinline__ C read(int i) const { return read_at(map(i)); }
-  __device__ __forceinline__ void write(int i, C v) const { write_at(map(i), v); }
-  __device__ __forceinline__ void sync() const { __syncthreads(); }
-};
-
-// Exchange for the column passes with a padded instead of a swizzled layout:
-// element i of FFT c at slot (i + (i >> L)) * CP + c, one pad slot per 2^L
+// interleaved element-wise in one CTA-wide SoA buffer, element i of FFT c at slot (i + (i >> L)) * CP + c, one pad slot per 2^L
 // elements (L = log2 RV).  With 32/CP consecutive transform threads per warp
 // the Stockham reads and writes, and the natural-order mid-point accesses,
 // fall in distinct banks, and every in-stage address folds into a

@@ -81,6 +81,8 @@ cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, in
 cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
                                    long long out_bs, int dtype, int dep, cudaStream_t st);
 
+// device table exp(-2 pi i k/n), k < n, or (rv > 0) its stage layout for rv values per thread
+int upload_twiddles(int n, int dtype, void** dev, int rv);
 // 1 unless `st` is being captured
 int dep_launches(cudaStream_t st);
 

@@ -18,34 +18,14 @@ struct fw_rho_plan {
   int N, batch, dtype;
   int nparts;           // row-pass CTAs per instance
   void* tw = nullptr;   // twiddles for length N
+  void* tws = nullptr;  // stage-layout twiddles of the row pass
+  float* gpf = nullptr; // FP32 copies of the p-observable kernels (RMAXO x N complex)
   double* ring = nullptr;
   int ring_M = 0;
 };
 
 namespace {
 constexpr int RHO_MMAX = 4 + 4 * RMAXO;
-
-int upload_tw(int n, int dtype, void** dev) {
-  std::vector<double> t(2 * (size_t)n);
-  for (int k = 0; k < n; ++k) {
-    const double a = -2.0 * M_PI * (double)k / (double)n;
-    t[2 * k] = cos(a);
-    t[2 * k + 1] = sin(a);
-  }
-  cudaError_t e;
-  if (dtype == FW_F64) {
-    e = cudaMalloc(dev, t.size() * sizeof(double));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(twiddles)");
-    e = cudaMemcpy(*dev, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice);
-  } else {
-    std::vector<float> f(t.begin(), t.end());
-    e = cudaMalloc(dev, f.size() * sizeof(float));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(twiddles)");
-    e = cudaMemcpy(*dev, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice);
-  }
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(twiddles)");
-  return FW_OK;
-}
 
 Factor to_factor(const fw_rho_factor* f) {
   Factor r{};
@@ -78,7 +58,12 @@ extern "C" int fw_rho_plan_create(int N, int batch, int dtype, fw_rho_plan** out
   p->batch = batch;
   p->dtype = dtype;
   p->nparts = rho_row_parts(dtype, N);
-  int rc = upload_tw(N, dtype, &p->tw);
+  int rc = upload_twiddles(N, dtype, &p->tw, 0);
+  if (rc == FW_OK) rc = upload_twiddles(N, dtype, &p->tws, rho_row_rv(dtype, N));
+  if (rc == FW_OK && dtype == FW_F32) {
+    cudaError_t e = cudaMalloc(&p->gpf, sizeof(float) * 2 * (size_t)RMAXO * N);
+    if (e != cudaSuccess) rc = cuda_fail(e, "cudaMalloc(observable kernels)");
+  }
   if (rc == FW_OK) {
     cudaError_t e = cudaMalloc(&p->ring, sizeof(double) * 2 * (size_t)batch * p->nparts * RHO_MMAX);
     if (e != cudaSuccess) rc = cuda_fail(e, "cudaMalloc(partials)");
@@ -94,6 +79,8 @@ extern "C" int fw_rho_plan_create(int N, int batch, int dtype, fw_rho_plan** out
 extern "C" int fw_rho_plan_destroy(fw_rho_plan* p) {
   if (p == nullptr) return FW_OK;
   cudaFree(p->tw);
+  cudaFree(p->tws);
+  cudaFree(p->gpf);
   cudaFree(p->ring);
   delete p;
   return FW_OK;
@@ -125,6 +112,7 @@ extern "C" int fw_rho_pass(fw_rho_plan* p, void* R, long long r_bstride, int axi
   a.part_out = part_out;
   a.sum_out = sum_out;
   a.tw = p->tw;
+  a.tws = p->tws;
   for (const fw_rho_factor* f : {f0, f1, f2, f3})
     if (f && f->on && f->shear_c != 0.0) { a.dX = f->shear_dx; a.dP = f->shear_dp; }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -186,6 +174,7 @@ extern "C" int fw_rho_propagate(fw_rho_plan* p, const fw_rho_desc* d, int steps,
   base.Mx = d->Mx;
   base.Mp = d->Mp;
   base.tw = p->tw;
+  base.tws = p->tws;
   base.dep = dep_launches(st);
   const double invN = 1.0 / (double)N;
   int np = 0;
@@ -201,6 +190,15 @@ extern "C" int fw_rho_propagate(fw_rho_plan* p, const fw_rho_desc* d, int steps,
     count_launch(1);
     return FW_OK;
   };
+  // kernels of static observables in the state precision, once per call
+  const void* gpr = nullptr;
+  if (p->dtype == FW_F32 && d->Mp > 0 && d->gp_step == 0) {
+    const int n = 2 * d->Mp * N;
+    cudaError_t e = launch_dep(base.dep, rho_gp_kernel, (n + 255) / 256, 256, 0, st, d->gp, n, p->gpf);
+    if (e != cudaSuccess) return cuda_fail(e, "rho observable kernels launch");
+    count_launch(1);
+    gpr = p->gpf;
+  }
   int rc;
   {
     RhoArgs a = base;  // opening expV of step 0, then FFT along x
@@ -225,6 +223,7 @@ extern "C" int fw_rho_propagate(fw_rho_plan* p, const fw_rho_desc* d, int steps,
     r.part_out = ring(k);
     r.wx = d->wx == nullptr ? nullptr : d->wx + (size_t)k * d->wx_step;
     r.gp = d->gp == nullptr ? nullptr : d->gp + (size_t)k * d->gp_step;
+    r.gpr = gpr;
     if (k + 1 < steps) {
       r.f2 = expV(k + 1, 1.0);
       r.t2 = -1;

@@ -45,8 +45,10 @@ struct RhoArgs {
   int Mx, Mp;
   const double* wx;    // Mx x N real (diagonal weights)
   const double* gp;    // Mp x N complex FP64 (G[(i - j) mod N])
+  const void* gpr;     // the same in the state precision, or null
   double* sum_out;     // if non-null: per-CTA complex sum of all elements after F3 (2 doubles)
-  const void* tw;
+  const void* tw;      // exp(-2 pi i k/N) (column passes)
+  const void* tws;     // stage-layout table of the row pass (fft.cuh, stage_off)
   int dep;  // programmatic dependent launch (launch_dep)
 };
 
@@ -82,23 +84,22 @@ __device__ __forceinline__ void rho_prev_scale(const RhoArgs& a, int b, double* 
   sim = 0.0;
   if (a.prev_part == nullptr) return;
   const double* pp = a.prev_part + (size_t)b * a.prev_nparts * a.M;
-  // lane-strided sums over the records and a fixed shuffle tree (deterministic,
-  // no serial chain through one thread); blockDim is a multiple of 32
+  // every thread takes records tid, tid + blockDim, ..., then a fixed tree
+  // (deterministic; one warp over all records waited on eight rounds of loads at
+  // 256 records); blockDim is a multiple of 32
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if (warp == 0) {
-    double tr = 0, ti = 0;
-    for (int c = lane; c < a.prev_nparts; c += 32) {
-      tr += pp[(size_t)c * a.M];
-      ti += pp[(size_t)c * a.M + 1];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      tr += __shfl_xor_sync(0xffffffffu, tr, o);
-      ti += __shfl_xor_sync(0xffffffffu, ti, o);
-    }
-    if (lane == 0) {
-      red[0] = tr;
-      red[1] = ti;
-    }
+  double tr = 0, ti = 0;
+  for (int c = threadIdx.x; c < a.prev_nparts; c += blockDim.x) {
+    tr += pp[(size_t)c * a.M];
+    ti += pp[(size_t)c * a.M + 1];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    ti += __shfl_xor_sync(0xffffffffu, ti, o);
+  }
+  if (lane == 0) {
+    red[2 * warp] = tr;
+    red[2 * warp + 1] = ti;
   }
   if (a.obs_hist != nullptr && blockIdx.x == 0) {  // one warp per record column
     for (int m = warp; m < a.M; m += nw) {
@@ -109,7 +110,13 @@ __device__ __forceinline__ void rho_prev_scale(const RhoArgs& a, int b, double* 
     }
   }
   __syncthreads();
-  const double tr = red[0] * a.dX, ti = red[1] * a.dX;
+  tr = ti = 0;
+  for (int w = 0; w < nw; ++w) {
+    tr += red[2 * w];
+    ti += red[2 * w + 1];
+  }
+  tr *= a.dX;
+  ti *= a.dX;
   const double d = tr * tr + ti * ti;
   sre = tr / d;
   sim = -ti / d;
@@ -156,27 +163,39 @@ __device__ __forceinline__ Factor pick_factor(bool s, const Factor& x, const Fac
 
 // forward (dir < 0) or unnormalised inverse (dir > 0) transform; the inverse is
 // conj(FFT(conj(x))) so each call site instantiates one transform.
-template <typename Rl, int N, int T, int RV, typename EX>
+template <typename Rl, int N, int T, int RV, bool STW, typename EX>
 __device__ __forceinline__ void transform(cplx_t<Rl> (&v)[RV], int dir, int j, EX& ex, const cplx_t<Rl>* tw) {
   if (dir == 0) return;
   if (dir > 0) {
 #pragma unroll
     for (int m = 0; m < RV; ++m) v[m].y = -v[m].y;
   }
-  fft<N, T, RV, -1>(v, j, ex, tw);
+  fft<N, T, RV, -1, cplx_t<Rl>, EX, STW>(v, j, ex, tw);
   if (dir > 0) {
 #pragma unroll
     for (int m = 0; m < RV; ++m) v[m].y = -v[m].y;
   }
 }
 
+// The exchange of one row's transform: complex slots where a warp owns it.
+template <typename Rl, int T> struct RowEx {
+  using EX = GroupEx<Rl, T>;
+  static __device__ __forceinline__ EX make(Rl* base, int buf, int g) { return EX{base, base + buf, 1 + g}; }
+};
+template <> struct RowEx<float, 32> {
+  using EX = GroupExC<float, 32>;
+  static __device__ __forceinline__ EX make(float* base, int, int) { return EX{reinterpret_cast<float2*>(base)}; }
+};
+
 // Row pass: G groups of T threads; group g owns row i.
-template <typename Rl, int N, int T, int G, int MINB, bool SH>
+// GPR: the p-observable kernels come from a.gpr (compile-time: a branch at every
+// load kept the loads from going out together, 37 -> 43 us per 1024^2 step).
+template <typename Rl, int N, int T, int G, int MINB, bool SH, bool GPR>
 __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
   using C = cplx_t<Rl>;
   constexpr int RV = N / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[4];
+  __shared__ double red[2 * (G * T / 32)];
   __shared__ double ored[G * T / 32][4 + 2 * (2 * RMAXO)];
   const int b = blockIdx.y;
   dep_sync();
@@ -185,9 +204,9 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
   const int i = blockIdx.x * G + g;
   constexpr int BUF = N + N / 32;
   Rl* base = reinterpret_cast<Rl*>(smem_raw) + (size_t)g * 2 * BUF;
-  GroupEx<Rl, T> ex{base, base + BUF, 1 + g};
+  auto ex = RowEx<Rl, T>::make(base, BUF, g);
   C* R = reinterpret_cast<C*>(a.R) + (size_t)b * a.r_bs + (size_t)i * N;
-  const C* tw = reinterpret_cast<const C*>(a.tw);
+  const C* tw = reinterpret_cast<const C*>(a.tws);
   C v[RV];
   // the loads go out before the scale's reduction
 #pragma unroll
@@ -205,7 +224,7 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
   for (int it = 0; it < 2; ++it) {
     const bool second = it != 0;
     apply_factor_row<Rl, N, T, RV, SH>(v, pick_factor(second, a.f0, a.f2), i, j, a.dX, a.dP, b);
-    transform<Rl, N, T, RV>(v, second ? a.t2 : a.t1, j, ex, tw);
+    transform<Rl, N, T, RV, true>(v, second ? a.t2 : a.t1, j, ex, tw);
     apply_factor_row<Rl, N, T, RV, SH>(v, pick_factor(second, a.f1, a.f3), i, j, a.dX, a.dP, b);
     if (!second && a.part_out != nullptr) {
       // [trace re, im, sum|rho|^2, 0, x-obs (re, im) x Mx, p-obs (re, im) x Mp]
@@ -237,8 +256,15 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
 #pragma unroll
         for (int q = 0; q < RMAXO; ++q)
           if (q < a.Mp) {
-            const double2 gk = __ldg(reinterpret_cast<const double2*>(a.gp) + (size_t)q * N + ((i - jj) & (N - 1)));
-            const Rl gx = (Rl)gk.x, gy = (Rl)gk.y;
+            const size_t gi = (size_t)q * N + ((i - jj) & (N - 1));
+            Rl gx, gy;
+            if constexpr (GPR) {
+              const C gk = __ldg(reinterpret_cast<const C*>(a.gpr) + gi);
+              gx = gk.x, gy = gk.y;
+            } else {
+              const double2 gk = __ldg(reinterpret_cast<const double2*>(a.gp) + gi);
+              gx = (Rl)gk.x, gy = (Rl)gk.y;
+            }
             pr[q] += re * gx - im * gy;
             pim[q] += re * gy + im * gx;
           }
@@ -249,20 +275,26 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
         acc[4 + 2 * RMAXO + 2 * q] = (double)pr[q];
         acc[5 + 2 * RMAXO + 2 * q] = (double)pim[q];
       }
-      // level-major warp reduction of the accumulators in use (acc[3] stays 0)
+      // reduce-scatter of the warp's accumulators: at each of the first levels a
+      // lane keeps half of its values and sends the other half, so twenty sums
+      // cost 16 + 8 + 4 + 2 + 1 shuffles of a double instead of 20 x 5 (the same
+      // tree of additions); lane l ends with value l (acc[3] stays 0)
+      static_assert(4 + 4 * RMAXO <= 32, "values per record");
+      const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+      double u[32];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+      for (int q = 0; q < 32; ++q) u[q] = q < 4 + 4 * RMAXO ? acc[q < 4 + 4 * RMAXO ? q : 0] : 0.0;
 #pragma unroll
-        for (int q = 0; q < 4 + 4 * RMAXO; ++q) {
-          const bool used = q < 3 || (q >= 4 && q < 4 + 2 * a.Mx) ||
-                            (q >= 4 + 2 * RMAXO && q < 4 + 2 * RMAXO + 2 * a.Mp);
-          if (used) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      for (int lv = 0; lv < 5; ++lv) {
+        const int off = 16 >> lv, half = 16 >> lv;
+        const bool up = (ln & off) != 0;
+#pragma unroll
+        for (int q = 0; q < half; ++q) {
+          const double send = up ? u[q] : u[q + half], keep = up ? u[q + half] : u[q];
+          u[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
-      const int warp = threadIdx.x >> 5;
-      if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int q = 0; q < 4 + 4 * RMAXO; ++q) ored[warp][q] = acc[q];
       }
+      if (ln < 4 + 4 * RMAXO) ored[warp][ln] = u[0];
       __syncthreads();
       if ((int)threadIdx.x < a.M) {
         const int mo = threadIdx.x;
@@ -299,20 +331,19 @@ __global__ void __launch_bounds__(G* T, MINB) rho_row_kernel(RhoArgs a) {
 }
 
 // Column pass: CP columns per CTA, T threads per column (interleaved exchange).
-template <typename Rl, int N, int T, int CP, int S, int MINB, bool SH>
+template <typename Rl, int N, int T, int CP, int MINB, bool SH>
 __global__ void __launch_bounds__(CP* T, MINB) rho_col_kernel(RhoArgs a) {
   using C = cplx_t<Rl>;
   constexpr int RV = N / T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[4];
+  __shared__ double red[2 * (CP * T / 32)];
   const int b = blockIdx.y;
   dep_sync();
   const int c = threadIdx.x % CP;
   const int jt = threadIdx.x / CP;
   __builtin_assume(jt >= 0 && jt < T);  // launched with exactly CP * T threads
   const int col = blockIdx.x * CP + c;
-  Rl* re = reinterpret_cast<Rl*>(smem_raw);
-  ColEx<Rl, CP, S> ex{re, re + (size_t)N * CP, c};
+  ColPadExC<Rl, CP, ilog2_c(RV)> ex{reinterpret_cast<C*>(smem_raw), c};
   C* R = reinterpret_cast<C*>(a.R) + (size_t)b * a.r_bs;
   const C* tw = reinterpret_cast<const C*>(a.tw);
   C v[RV];
@@ -325,27 +356,32 @@ __global__ void __launch_bounds__(CP* T, MINB) rho_col_kernel(RhoArgs a) {
 #pragma unroll
   for (int m = 0; m < RV; ++m) v[m] = cmul(v[m], sc);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f0, jt, col, a.dX, a.dP, b);
-  transform<Rl, N, T, RV>(v, a.t1, jt, ex, tw);
+  transform<Rl, N, T, RV, false>(v, a.t1, jt, ex, tw);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f1, jt, col, a.dX, a.dP, b);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f2, jt, col, a.dX, a.dP, b);
-  transform<Rl, N, T, RV>(v, a.t2, jt, ex, tw);
+  transform<Rl, N, T, RV, false>(v, a.t2, jt, ex, tw);
   apply_factor_col<Rl, N, T, RV, SH>(v, a.f3, jt, col, a.dX, a.dP, b);
 #pragma unroll
   for (int m = 0; m < RV; ++m) R[(size_t)(jt + m * T) * N + col] = v[m];
 }
 
 // ---------------------------------------------------------------------------
+// Launch shapes.  At 512 two CTAs per SM of half the columns (FP64 also rows) beat
+// one of threads that hold everything: 22.9 -> 20.1 us a step in FP32, 26.4 -> 23.3 in
+// FP64; at 1024 FP32 the 512-thread column CTAs are the faster ones (37.8 against
+// 41 to 55 us for smaller tiles, all before the exchanges and reductions of this
+// file were changed: 39.5 us a step, now 31.2).
 template <typename Rl, int N> struct RhoRowCfg;
 template <typename Rl, int N> struct RhoColCfg;
 #define RCFG(R, N_, T_, G_, MB_) template <> struct RhoRowCfg<R, N_> { static constexpr int T = T_, G = G_, MINB = MB_; };
 #define CCFG(R, N_, T_, CP_, MB_) template <> struct RhoColCfg<R, N_> { static constexpr int T = T_, CP = CP_, MINB = MB_; };
 RCFG(float, 128, 16, 8, 1) RCFG(float, 256, 32, 4, 2) RCFG(float, 512, 32, 4, 2) RCFG(float, 1024, 32, 4, 2)
 RCFG(float, 2048, 64, 4, 1) RCFG(float, 4096, 128, 2, 1)
-RCFG(double, 128, 16, 8, 1) RCFG(double, 256, 16, 8, 1) RCFG(double, 512, 32, 4, 1) RCFG(double, 1024, 64, 2, 1)
+RCFG(double, 128, 16, 8, 1) RCFG(double, 256, 16, 8, 1) RCFG(double, 512, 32, 4, 2) RCFG(double, 1024, 64, 2, 1)
 RCFG(double, 2048, 128, 2, 1) RCFG(double, 4096, 256, 1, 1)
-CCFG(float, 128, 16, 16, 1) CCFG(float, 256, 32, 16, 1) CCFG(float, 512, 32, 16, 1) CCFG(float, 1024, 64, 8, 1)
+CCFG(float, 128, 16, 16, 1) CCFG(float, 256, 32, 16, 1) CCFG(float, 512, 32, 8, 2) CCFG(float, 1024, 64, 8, 1)
 CCFG(float, 2048, 64, 8, 1) CCFG(float, 4096, 128, 4, 1)
-CCFG(double, 128, 16, 8, 1) CCFG(double, 256, 16, 8, 1) CCFG(double, 512, 32, 8, 1) CCFG(double, 1024, 64, 4, 1)
+CCFG(double, 128, 16, 8, 1) CCFG(double, 256, 16, 8, 1) CCFG(double, 512, 32, 4, 2) CCFG(double, 1024, 64, 4, 1)
 CCFG(double, 2048, 128, 2, 1) CCFG(double, 4096, 256, 2, 1)
 #undef RCFG
 #undef CCFG
@@ -354,12 +390,12 @@ static bool any_shear(const RhoArgs& a) {
   return a.f0.shear_c != 0.0 || a.f1.shear_c != 0.0 || a.f2.shear_c != 0.0 || a.f3.shear_c != 0.0;
 }
 
-template <typename Rl, int N, bool SH>
+template <typename Rl, int N, bool SH, bool GPR>
 static cudaError_t rho_row_sh(const RhoArgs& a, cudaStream_t st, int* nparts) {
   using Cfg = RhoRowCfg<Rl, N>;
   constexpr int T = Cfg::T, G = Cfg::G, MINB = Cfg::MINB;
   const size_t smem = (size_t)G * 2 * (N + N / 32) * sizeof(Rl);
-  auto kern = rho_row_kernel<Rl, N, T, G, MINB, SH>;
+  auto kern = rho_row_kernel<Rl, N, T, G, MINB, SH, GPR>;
   static PerDeviceOnce attr;  // per device: the attribute is set on the device current at the call
   cudaError_t e = set_smem_once(attr, kern, smem);
   if (e != cudaSuccess) return e;
@@ -372,16 +408,19 @@ static cudaError_t rho_row_sh(const RhoArgs& a, cudaStream_t st, int* nparts) {
 // with the per-element sincos; propagation passes carry none of that code.
 template <typename Rl, int N>
 static cudaError_t rho_row_n(const RhoArgs& a, cudaStream_t st, int* nparts) {
-  return any_shear(a) ? rho_row_sh<Rl, N, true>(a, st, nparts) : rho_row_sh<Rl, N, false>(a, st, nparts);
+  if (any_shear(a)) return rho_row_sh<Rl, N, true, false>(a, st, nparts);
+  if constexpr (sizeof(Rl) == 4) {
+    if (a.gpr != nullptr) return rho_row_sh<Rl, N, false, true>(a, st, nparts);
+  }
+  return rho_row_sh<Rl, N, false, false>(a, st, nparts);
 }
 
 template <typename Rl, int N, bool SH>
 static cudaError_t rho_col_sh(const RhoArgs& a, cudaStream_t st) {
   using Cfg = RhoColCfg<Rl, N>;
   constexpr int T = Cfg::T, CP = Cfg::CP, MINB = Cfg::MINB;
-  constexpr int S = ilog2_c(N / T > 32 ? 32 : N / T);
-  const size_t smem = (size_t)2 * N * CP * sizeof(Rl);
-  auto kern = rho_col_kernel<Rl, N, T, CP, S, MINB, SH>;
+  const size_t smem = (size_t)2 * (N + T) * CP * sizeof(Rl);  // one pad slot per N / T elements
+  auto kern = rho_col_kernel<Rl, N, T, CP, MINB, SH>;
   static PerDeviceOnce attr;  // per device: the attribute is set on the device current at the call
   cudaError_t e = set_smem_once(attr, kern, smem);
   if (e != cudaSuccess) return e;
@@ -392,6 +431,23 @@ static cudaError_t rho_col_sh(const RhoArgs& a, cudaStream_t st) {
 template <typename Rl, int N>
 static cudaError_t rho_col_n(const RhoArgs& a, cudaStream_t st) {
   return any_shear(a) ? rho_col_sh<Rl, N, true>(a, st) : rho_col_sh<Rl, N, false>(a, st);
+}
+
+// the p-observable kernels in FP32
+__global__ void rho_gp_kernel(const double* gp, int n, float* out) {
+  dep_sync();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (float)gp[i];
+}
+
+// Values per thread of the row pass transform (its stage-layout twiddles).
+int rho_row_rv(int dtype, int N) {
+  int t = 0;
+#define RV_(R, N_) if (N == N_) t = RhoRowCfg<R, N_>::T;
+  if (dtype == FW_F32) { RV_(float, 128) RV_(float, 256) RV_(float, 512) RV_(float, 1024) RV_(float, 2048) RV_(float, 4096) }
+  else { RV_(double, 128) RV_(double, 256) RV_(double, 512) RV_(double, 1024) RV_(double, 2048) RV_(double, 4096) }
+#undef RV_
+  return t == 0 ? 0 : N / t;
 }
 
 int rho_row_parts(int dtype, int N) {
