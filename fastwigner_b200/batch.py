@@ -354,27 +354,53 @@ class WignerMoyalUnevenBatch:
         self.t += steps * self.dt
         return obs
 
-    def _launch_groups(self, steps, obs, obs_g):
+    def _launch_group(self, g, og, steps):
         from ._lib import FW_STEP_FUSED
 
-        # the groups one after another on the current stream: replayed from a
-        # graph, the small groups' launches are short enough that side streams
-        # gained nothing over this order (0.669 vs 0.668 ms per step for the
-        # 256-instance mix of 16 shapes) and a multi-stream graph lost 17 %
-        for g, og in zip(self._groups, obs_g):
-            d = WignerDesc()
-            d.W = ptr(g["W"])
-            d.w_bstride = g["P"] * g["X"]
-            d.step_kind = FW_STEP_FUSED
-            d.tabV, d.tabK = ptr(g["tab"][0]), ptr(g["tab"][1])
-            d.tab_bstride = 2 * g["S"]
-            d.obs_out = ptr(og)
-            d.dxdp = g["dxdp"]
-            d.in_scale = 1.0
-            check(self._lib.fw_wigner_propagate(g["plan"], ctypes.byref(d), steps, stream_handle()),
-                  "fw_wigner_propagate")
+        d = WignerDesc()
+        d.W = ptr(g["W"])
+        d.w_bstride = g["P"] * g["X"]
+        d.step_kind = FW_STEP_FUSED
+        d.tabV, d.tabK = ptr(g["tab"][0]), ptr(g["tab"][1])
+        d.tab_bstride = 2 * g["S"]
+        d.obs_out = ptr(og)
+        d.dxdp = g["dxdp"]
+        d.in_scale = 1.0
+        check(self._lib.fw_wigner_propagate(g["plan"], ctypes.byref(d), steps, stream_handle()),
+              "fw_wigner_propagate")
+
+    def _launch_groups(self, steps, obs, obs_g, lanes=1):
+        """Every group's steps, then the observables in instance order.  lanes > 1
+        (under capture): the groups, largest first, in that many parallel branches
+        of the graph."""
+        if lanes <= 1:
+            for g, og in zip(self._groups, obs_g):
+                self._launch_group(g, og, steps)
+        else:
+            main = torch.cuda.current_stream(self.device)
+            side = [torch.cuda.Stream(self.device) for _ in range(lanes)]
+            load = [0] * lanes
+            for s in side:
+                s.wait_stream(main)
+            order = sorted(range(len(self._groups)), key=lambda i: -self._groups[i]["W"].numel())
+            for i in order:
+                k = load.index(min(load))
+                load[k] += self._groups[i]["W"].numel() + (1 << 18)  # a chain's latency, in points
+                with torch.cuda.stream(side[k]):
+                    self._launch_group(self._groups[i], obs_g[i], steps)
+            for s in side:
+                main.wait_stream(s)
         for g, og in zip(self._groups, obs_g):
             obs.index_copy_(1, g["idx_t"], og)
+
+    def _lanes(self):
+        """Parallel branches of the captured graph: a group's launches are a chain of
+        kernels of a few microseconds that fill part of the GPU, so chains run
+        side by side, fewer of them the larger the states are (us per step one
+        after another / in parallel: 6 instances 98 / 32, 24: 262 / 106, 48: 283 / 168
+        to 192, 96: 352 / 249, 256: 594 / 496 with two branches, 544 with four)."""
+        pts = sum(g["W"].numel() for g in self._groups)
+        return max(1, min(len(self._groups), 8, max(2, 50_000_000 // pts)))
 
     def _propagate_grouped(self, steps, use_graph, obs):
         if not use_graph:
@@ -391,7 +417,7 @@ class WignerMoyalUnevenBatch:
             torch.cuda.synchronize(self.device)
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
-                self._launch_groups(steps, obs, obs_g)
+                self._launch_groups(steps, obs, obs_g, self._lanes())
             self._graph, self._graph_key, self._graph_obs = graph, key, obs_g
             # the direct call above already advanced the states by `steps`
             return
