@@ -21,7 +21,7 @@
 // transform's multiply-adds for sizes with a large prime factor.  Against one
 // pair per CTA, radix 4/2/3/5 stages only, every other prime as one thread's
 // direct sum and unfused column half-steps: 8 x 600 x 1000 FP32, 10 steps,
-// 3.93 -> 1.55 ms; one 98 x 202 FP64 object, 10 steps, 42.7 -> 0.35 ms.
+// 3.93 -> 1.13 ms; one 98 x 202 FP64 object, 10 steps, 42.7 -> 0.34 ms.
 #include "fw_internal.h"
 #include "wigner_tiles.cuh"
 
@@ -29,6 +29,12 @@ namespace fw {
 
 constexpr int kGenThreads = 256;
 constexpr int kGenMaxStages = 12;
+// CTAs per SM the passes are compiled for, and the shared memory of one that
+// lets as many be resident: the stages wait on shared memory and barriers, so FP32
+// runs four CTAs of 64 registers (8 x 600 x 1000: 146 us a step with two, 118 with three,
+// 106 with four; 8 x 300 x 900: 104, 81, 59), FP64, which would spill, two.
+template <typename Rl> __host__ __device__ constexpr int gen_minb() { return sizeof(Rl) == 4 ? 4 : 2; }
+constexpr size_t kGenSmem32 = (size_t)56 << 10, kGenSmem64 = (size_t)110 << 10;
 // FP32 direct transforms of primes above this sum their terms in index order
 // (gen_sequential) and keep the two potential half-steps on transform pairs of
 // their own.  The rounding of such long FP32 sums is the same function of the
@@ -444,7 +450,7 @@ template <int NV> __device__ __forceinline__ void gen_block_sum(double (&v)[NV],
 }
 
 template <typename Rl>
-__global__ void __launch_bounds__(kGenThreads, 2) gen_row_kernel(PassArgs a, GenFactors g, int lcp) {
+__global__ void __launch_bounds__(kGenThreads, gen_minb<Rl>()) gen_row_kernel(PassArgs a, GenFactors g, int lcp) {
   using C = cplx_t<Rl>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[34];
@@ -487,7 +493,7 @@ __global__ void __launch_bounds__(kGenThreads, 2) gen_row_kernel(PassArgs a, Gen
 // mid-point (mask, blend, observables), or (fuse_mid) two on one transform
 // pair with the observables from the mid-point spectrum.
 template <typename Rl>
-__global__ void __launch_bounds__(kGenThreads, 2) gen_col_kernel(PassArgs a, GenFactors g, int lcp) {
+__global__ void __launch_bounds__(kGenThreads, gen_minb<Rl>()) gen_col_kernel(PassArgs a, GenFactors g, int lcp) {
   using C = cplx_t<Rl>;
   using V2 = typename Vec2<Rl>::type;
   constexpr int NV = 2 + 2 * MAXO;  // sum, sum of squares, x-weights, p-weights
@@ -705,14 +711,15 @@ template <typename C> static size_t gen_smem(int N, int lcp) {
 }
 
 // Pairs per CTA (as a power of two, the exponent): enough that a row of the
-// tile fills the 32-byte sectors it touches, as long as two CTAs fit an SM and
-// the launch has two CTAs per SM.
+// tile fills the sectors it touches, as long as the CTAs of gen_minb fit an SM
+// and the launch has two CTAs per SM (4 x 1000 x 1000 FP32: 101 us a step with
+// two pairs and four CTAs, 112 with four pairs and two CTAs).
 static int gen_lcp(int dtype, int N, int pairs, int batch) {
   auto smem = [&](int l) { return dtype == FW_F64 ? gen_smem<double2>(N, l) : gen_smem<float2>(N, l); };
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int l = dtype == FW_F64 ? 1 : 2;
-  while (l > 0 && (smem(l) > (size_t)100 << 10 ||
+  int l = dtype == FW_F64 ? 2 : 3;
+  while (l > 0 && (smem(l) > (dtype == FW_F64 ? kGenSmem64 : kGenSmem32) ||
                    (long long)((pairs + (1 << l) - 1) >> l) * batch < 2LL * sms))
     --l;
   return l;
