@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(256, 2) project_bwd_kernel(long long L, int ba
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float u = h[i][k] + b1[i];
-          s2 = fmaf(gelu(u), x[k], s2);
-          h[i][k] = w2[i] * x[k] * gelu_d(u);
+          s2 = fmaf(gelu_tail(u), x[k], s2);
+          h[i][k] = w2[i] * x[k] * gelu_d_tail(u);
           sc += h[i][k];
         }
         gc[i] += (double)sc;

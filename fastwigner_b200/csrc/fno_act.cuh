@@ -1,7 +1,6 @@
-// GELU and its derivative, shared by the FNO's element-wise kernels and the
-// tensor-core epilogues so that fused and unfused paths round alike.
+// GELU and its derivative for the FNO's kernels, in two forms.
 //
-// GELU(x) = x Phi(x) with the lower tail q = Phi(-|x|) = exp(-x^2/2) R(|x|): the
+// The fused kernels: GELU(x) = x Phi(x) with the lower tail q = Phi(-|x|) = exp(-x^2/2) R(|x|): the
 // scaled tail R is a polynomial in t = 1/(1 + 0.28 |x|) (the form of Hastings'
 // error-function approximations), fitted here by iteratively reweighted least
 // squares to 9e-9 absolute in q.  No branches: about 16 instructions, two of
@@ -25,8 +24,13 @@ __device__ __forceinline__ void gauss_tail(float x, float& q, float& e) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -0.72134752044448169f * x));
   q = p * t * e;
 }
+// The erff forms, of the unfused kernels: the training forward pass runs them.
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_d(float x) {
+  return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
 // x Phi(x) = max(x, 0) - |x| q; the clamp keeps an infinite x from 0 * inf
-__device__ __forceinline__ float gelu(float x) {
+__device__ __forceinline__ float gelu_tail(float x) {
   float q, e;
   gauss_tail(x, q, e);
   return fmaf(-fminf(fabsf(x), 3.4e38f), q, fmaxf(x, 0.f));
@@ -52,7 +56,7 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// gelu of two values, operation for operation
+// gelu_tail of two values, operation for operation
 __device__ __forceinline__ void gelu2(float& x, float& y) {
   const float ax = fabsf(x), ay = fabsf(y);
   float dx, dy, ex, ey;
@@ -70,7 +74,7 @@ __device__ __forceinline__ void gelu2(float& x, float& y) {
   const uint64_t q = mul2(mul2(p, t), pack2(ex, ey));
   unpack2(fma2(pack2(-fminf(ax, 3.4e38f), -fminf(ay, 3.4e38f)), q, pack2(fmaxf(x, 0.f), fmaxf(y, 0.f))), x, y);
 }
-__device__ __forceinline__ float gelu_d(float x) {
+__device__ __forceinline__ float gelu_d_tail(float x) {
   float q, e;
   gauss_tail(x, q, e);
   return fmaf(x * 0.39894228040143268f, e, x >= 0.f ? 1.f - q : q);

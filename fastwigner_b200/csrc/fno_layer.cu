@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) x[i] = st < nx ? __ldg(p + (h + i) * chs) : 0.f;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[h + i] *= gelu_d(x[i]);
+          for (int i = 0; i < 16; ++i) v[h + i] *= gelu_d_tail(x[i]);
         }
       }
     } else {
