@@ -102,7 +102,7 @@ _SIGNATURES = [
     ("fw_fno_project_bwd_work", c_int, [c_ll, c_int, ctypes.POINTER(c_ll)]),
     ("fw_fno_project_bwd", c_int, [c_ll, c_int, c_vp, c_ll] + [c_vp] * 6 + [c_ll] + [c_vp] * 5),
     ("fw_fno_project", c_int, [c_int, c_int, c_ll, c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp]),
-    ("fw_fno_layer", c_int, [c_int] * 4 + [c_vp] * 6 + [c_int] * 2 + [c_vp] * 14),
+    ("fw_fno_layer", c_int, [c_int] * 4 + [c_vp] * 6 + [c_int] * 2 + [c_vp] * 13),
     ("fw_fno_pdft", c_int, [c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     ("fw_fno_pidft", c_int, [c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     ("fw_fno_thermal", c_int, [c_int] * 3 + [c_vp] * 3 + [ctypes.c_double] * 2 + [c_vp] * 3),

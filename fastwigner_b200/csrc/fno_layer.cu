@@ -91,8 +91,8 @@ struct LayerArgs {
   const float *Q1, *c1, *Q2, *c2;  // LAST
   float* out;          // LAST: [rows][G1]
   int rows, G1, tiles, act;  // act: 0 none, 1 GELU, 2 times GELU'(aux)
-  const float* aux;     // channel-major [b][32][G0][G1], as the three below; LIFT: v' is read from it instead
-  float *pre, *vcm;     // optional copies of the pre-activation and of v'
+  const float* aux;     // channel-major [b][32][G0][G1], as vcm; LIFT: v' is read from it instead
+  float* vcm;           // MID: optional copy of v'
 };
 
 // float index of element (row, k) of a 128-byte-row, 128-byte-swizzled tile
@@ -325,11 +325,6 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       tmem_ld64(trow + D1_COL + 64, t);
 #pragma unroll
       for (int i = 0; i < LC; ++i) v[i] = v[i] + (t[i] + t[32 + i]) + s_bias[i];
-      if (MODE == LAYER_MID && a.pre != nullptr && st < nx) {
-        float* p = a.pre + cm_base(r);
-#pragma unroll
-        for (int i = 0; i < LC; ++i) p[i * chs] = v[i];
-      }
       if (a.act == 1) {
 #pragma unroll
         for (int i = 0; i < LC; i += 2) gelu2(v[i], v[i + 1]);
@@ -368,7 +363,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
 #pragma unroll
       for (int i = 0; i < LC; ++i) v[i] = 0.f;
     }
-    if (a.vcm != nullptr && st < nx) {
+    if (MODE == LAYER_MID && a.vcm != nullptr && st < nx) {
       float* p = a.vcm + cm_base(r);
 #pragma unroll
       for (int i = 0; i < LC; ++i) p[i * chs] = v[i];
@@ -705,8 +700,7 @@ using namespace fw::fnol;
 extern "C" int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float* gx, const float* AA,
                             const float* CS, const float* W, const float* bias, int act, int NP, const float* par,
                             const float* xs, const float* ps, const float* Q1, const float* c1, const float* Q2, const float* c2,
-                            float* vout, float* fx, float* out, const float* aux, float* pre, float* vcm,
-                            void* stream) {
+                            float* vout, float* fx, float* out, const float* aux, float* vcm, void* stream) {
   if (int rc = check_dims(B, G0, G1, "fw_fno_layer")) return rc;
   if (mode < LAYER_LIFT || mode > LAYER_LAST) return fail(FW_EINVAL, "fw_fno_layer: mode must be 0, 1 or 2");
   const bool copy = mode == LAYER_LIFT && aux != nullptr;
@@ -719,15 +713,16 @@ extern "C" int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, c
                          : (!on16(vin) || !on16(gx) || AA == nullptr))
     return fail(FW_EINVAL, "fw_fno_layer: NULL input, or activations off 16 bytes");
   if (mode == LAYER_LAST ? (Q1 == nullptr || c1 == nullptr || Q2 == nullptr || c2 == nullptr || out == nullptr)
-      : fx == nullptr    ? (vcm == nullptr || vout != nullptr)
+      : fx == nullptr    ? (mode != LAYER_MID || vcm == nullptr || vout != nullptr)
                          : (!on16(vout) || CS == nullptr))
     return fail(FW_EINVAL, "fw_fno_layer: NULL output, or activations off 16 bytes");
+  if (vcm != nullptr && mode != LAYER_MID) return fail(FW_EINVAL, "fw_fno_layer: vcm is mode 1's");
   LayerArgs a{};
   a.vin = vin, a.gx = gx, a.AA = AA, a.CS = CS, a.W = W, a.bias = bias, a.act = act;
   a.NP = NP, a.par = par, a.xs = xs, a.ps = ps, a.G0 = G0;
   if (int rc = fno_status_ptr(&a.status)) return rc;
   a.vout = vout, a.fx = fx, a.Q1 = Q1, a.c1 = c1, a.Q2 = Q2, a.c2 = c2, a.out = out;
-  a.aux = aux, a.pre = pre, a.vcm = vcm;
+  a.aux = aux, a.vcm = vcm;
   a.rows = B * G0, a.G1 = G1, a.tiles = (G1 + LX - 1) / LX;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = mode == LAYER_LIFT  ? launch_layer<LAYER_LIFT>(a, st)

@@ -85,11 +85,11 @@ class _Ops:
                                       stream_handle()), "fw_fno_project")
 
     def layer(self, mode, B, G0, G1, W, bias, act=0, vin=None, gx=None, AA=None, CS=None, NP=0, par=None, xs=None,
-              ps=None, Q1=None, c1=None, Q2=None, c2=None, vout=None, fx=None, out=None, aux=None, pre=None, vcm=None):
+              ps=None, Q1=None, c1=None, Q2=None, c2=None, vout=None, fx=None, out=None, aux=None, vcm=None):
         opt = lambda t: _p(t) if t is not None else None
         check(self.lib.fw_fno_layer(mode, B, G0, G1, opt(vin), opt(gx), opt(AA), opt(CS), opt(W), opt(bias), int(act),
                                     NP, opt(par), opt(xs), opt(ps), opt(Q1), opt(c1), opt(Q2), opt(c2), opt(vout),
-                                    opt(fx), opt(out), opt(aux), opt(pre), opt(vcm), stream_handle()), "fw_fno_layer")
+                                    opt(fx), opt(out), opt(aux), opt(vcm), stream_handle()), "fw_fno_layer")
 
     def thermal(self, out, wc, xs, ps, x_e, dxdp):
         """Thermal states from network outputs (in place), see fw_fno_thermal."""

@@ -378,15 +378,15 @@ int fw_fno_project(int hidden, int C, long long L, const float* V, long long str
  * v[b][g0][x][32], the eight 16-byte pieces of pixel x at positions piece ^ (x & 7); vin may be vout; 16-byte aligned.
  * mode 0: v = lift of (par[b][0..NP), xs[x], ps[g0]) with W 32 x (NP + 2); mode 1: v' = act(AA^T gx + W v + bias);
  * mode 2: the same, then out = Q2 GELU(Q1 v' + c1) + c2 (128 hidden) and nothing else.  Modes 0 and 1 also write fx, the
- * forward x-transform of v' (CS: G1 x 32) per 128-pixel tile: [ceil(G1/128)][B G0][32 channels][32 parts]; with fx (and
- * vout) NULL only the channel-major copies.  Channel-major arrays, [B][32][G0][G1], for training: vcm (v'), pre (the
- * pre-activation, mode 1; vcm in mode 2 too); aux: act 2 multiplies by GELU'(aux) (a layer's backward: CS^T and AA^T for AA and CS, W^T for
- * W), and mode 0 with aux copies it instead of lifting.
+ * forward x-transform of v' (CS: G1 x 32) per 128-pixel tile: [ceil(G1/128)][B G0][32 channels][32 parts].  For a
+ * layer's backward (CS^T and AA^T for AA and CS, W^T for W), with channel-major arrays [B][32][G0][G1]: mode 1 copies v'
+ * to vcm (and writes nothing else with fx and vout NULL), its act 2 multiplies by GELU'(aux); mode 0 with aux copies it
+ * instead of lifting.
  * G0 in [32, 1024], G1 >= 32 a multiple of 4, NP <= 14. */
 int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float* gx, const float* AA, const float* CS,
                  const float* W, const float* bias, int act, int NP, const float* par, const float* xs, const float* ps,
                  const float* Q1, const float* c1, const float* Q2, const float* c2, float* vout, float* fx, float* out,
-                 const float* aux, float* pre, float* vcm, void* stream);
+                 const float* aux, float* vcm, void* stream);
 /* F2[b][c][2][32 x 16] = p-transform of fx (tiles summed); gx[b][p][c][32 parts] (swizzled rows) = inverse
  * p-transform of O2.  Dpv, Dpiv: the interleaved DFT matrices (64 x 2 G0, 2 G0 x 64). */
 int fw_fno_pdft(int B, int G0, int G1, const float* fx, const float* Dpv, float* F2, void* stream);
