@@ -99,7 +99,7 @@ def test_weight_and_bias_gradients(rows, cols, L, B):
 
 @pytest.mark.parametrize("G0,G1,B", [(32, 36, 1), (48, 192, 2), (64, 132, 3)])
 def test_training_gradients_match_autograd(G0, G1, B):
-    """One loss_and_grad + backward on the fused path (layers both ways, projection
+    """One loss_and_grad + backward on the fused path (layers' and projection
     backward, weight gradients) against FP64 autograd, 2e-5 of each gradient's
     maximum (a gradient is a chain of about ten products of 1e-6 each)."""
     from fastwigner_b200.fno import FNO2d
