@@ -192,11 +192,11 @@ class StrongFieldWigner(WignerMoyalFTTW1D):
         """exp(i c f_k y) over steps k and grid points y, steps x len x 2: the
         phases in FP64 on the device, rounded once (as complex exponentials on the
         host the 64 x 1025 factors of a chunk took 2.4 ms, longer than the chunk
-        runs)."""
-        y = getattr(self, "_factor_grid", None)
-        if y is None:
-            y = self._factor_grid = to_device(grid.reshape(-1), torch.float64, self.device)
-        ph = torch.outer(torch.from_numpy(np.ascontiguousarray(f, dtype=np.float64)).to(self.device), y).mul_(c)
+        runs).  The axis travels with the field values in one upload: the gauge, and
+        with it the axis, may change between calls."""
+        f = np.asarray(f, dtype=np.float64).reshape(-1)
+        d = torch.from_numpy(np.concatenate([f, np.asarray(grid, dtype=np.float64).reshape(-1)])).to(self.device)
+        ph = torch.outer(d[:f.size], d[f.size:]).mul_(c)
         return torch.stack([torch.cos(ph), torch.sin(ph)], dim=-1).to(self._rt).contiguous()
 
     def _propagate_chunk(self, nsteps, t0, tables=None, weights=None, host=True):
