@@ -520,7 +520,7 @@ int noalloc_layout(int P, int X, int batch, int dtype, const fw_wigner_desc* d, 
   if (L->np <= 0) return fail(FW_EINVAL, "fw_wigner_propagate_noalloc: unsupported X for the column pass tile");
   const size_t rs = dtype == FW_F64 ? sizeof(double) : sizeof(float);
   L->rvX = row_rv(dtype, X, L->small);
-  L->nsX = stage_off(X, L->rvX, X);
+  L->nsX = L->rvX > 0 ? stage_off(X, L->rvX, X) : 0;  // (the generic row pass reads the k-indexed table)
   // p-weight spectra (fused mid-point column pass): shared or per-instance weights
   const bool pw = d != nullptr && d->Mp > 0;
   L->wph_nb = pw ? (d->wp_bstride != 0 ? batch : 1) : 0;
@@ -590,7 +590,7 @@ extern "C" int fw_wigner_propagate_noalloc(int P, int X, int batch, int dtype, c
   tmp.small = L.small;
   tmp.twP = base + L.twP;
   tmp.twX = base + L.twX;
-  tmp.twsX = base + L.twsX;
+  tmp.twsX = base + (L.nsX > 0 ? L.twsX : L.twX);
   tmp.ring = reinterpret_cast<double*>(base + L.ring);
   tmp.tot = reinterpret_cast<double*>(base + L.tot);
   tmp.wph = L.wph_nb > 0 ? base + L.wph : nullptr;
