@@ -302,10 +302,15 @@ extern "C" int fw_wigner_propagate(fw_wigner_plan* plan, const fw_wigner_desc* d
       if (d->wp_step != 0 || plan->wph == nullptr || nb > plan->wph_nb) {
         fuse = false;
       } else {
+        // entries per instance: P bins of 4 in the state's precision, or the
+        // generic pass's P/2 of 4 in FP64 (no more bytes)
+        const bool gen = col_generic(plan->dtype, plan->P, plan->X);
+        const long long bs = (gen ? 2LL : 4LL) * plan->P;
         base.wph = plan->wph;
-        base.wph_bs = d->wp_bstride != 0 ? 4LL * plan->P : 0;
-        cudaError_t e = launch_pweight_dft(d->wp, d->wp_bstride, d->Mp, plan->P, nb, plan->wph, 4LL * plan->P,
-                                           plan->dtype, base.dep, st);
+        base.wph_bs = d->wp_bstride != 0 ? bs : 0;
+        cudaError_t e = gen ? launch_generic_pweight(d->wp, d->wp_bstride, d->Mp, plan->P, nb, plan->wph, bs, base.dep, st)
+                            : launch_pweight_dft(d->wp, d->wp_bstride, d->Mp, plan->P, nb, plan->wph, bs, plan->dtype,
+                                                 base.dep, st);
         if (e != cudaSuccess) return cuda_fail(e, "weight spectrum launch");
         ++g_launches;
       }

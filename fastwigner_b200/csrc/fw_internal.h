@@ -75,11 +75,10 @@ int small_shapes(int dtype, int P, int X, int batch);
 bool size_supported(int n);
 bool size_pow2_supported(int n);
 bool col_generic(int dtype, int P, int X);
-inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 cudaError_t launch_generic_row(const PassArgs& a, int dtype, cudaStream_t st);
 cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, int* nparts);
 cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
-                                   long long out_bs, int dtype, int dep, cudaStream_t st);
+                                   long long out_bs, int dep, cudaStream_t st);
 
 // device table exp(-2 pi i k/n), k < n, or (rv > 0) its stage layout for rv values per thread
 int upload_twiddles(int n, int dtype, void** dev, int rv);

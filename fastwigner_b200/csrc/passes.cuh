@@ -64,7 +64,9 @@ struct PassArgs {
   double out_scale;
   int* status;  // device status word (error flags); may be null
   int fuse_mid;
-  const void* wph;  // complex, same precision as W, [b][k][4] (bin-major, 4 weights per bin)
+  // complex, same precision as W, [b][k][4] (bin-major, 4 weights per bin); for the
+  // generic passes FP64 [b][q][k], as gen_pweight_kernel writes it
+  const void* wph;
   long long wph_bs;
   int tab_vec;      // tab1/tab2 start on 16 bytes: a column pair's two entries load as one vector
   // Per-instance totals of the previous pass's partial sums (reduced by

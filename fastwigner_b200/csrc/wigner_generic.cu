@@ -21,7 +21,8 @@
 // transform's multiply-adds for sizes with a large prime factor.  Against one
 // pair per CTA, radix 4/2/3/5 stages only, every other prime as one thread's
 // direct sum and unfused column half-steps: 8 x 600 x 1000 FP32, 10 steps,
-// 3.93 -> 1.13 ms; one 98 x 202 FP64 object, 10 steps, 42.7 -> 0.34 ms.
+// 3.93 -> 1.14 ms (1.13 with FP32 squares and weight spectra, which narrowed the
+// observables); one 98 x 202 FP64 object, 10 steps, 42.7 -> 0.34 ms.
 #include "fw_internal.h"
 #include "wigner_tiles.cuh"
 
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(kGenThreads, gen_minb<Rl>()) gen_col_kernel(Pa
     }
   };
   if (a.fuse_mid) {
-    const C* G = reinterpret_cast<const C*>(a.wph) + (size_t)b * a.wph_bs;
+    const double2* G = reinterpret_cast<const double2*>(a.wph) + (size_t)b * a.wph_bs;
     const bool same = a.tab1 == a.tab2 && a.g1 == a.g2;
     gen_fill(z, N, lcp, load);
     gen_fft<-1>(z, z2, N, g, lcp, tw);
@@ -585,15 +586,17 @@ __global__ void __launch_bounds__(kGenThreads, gen_minb<Rl>()) gen_col_kernel(Pa
       A = cmul(A, ea);   // 2 x the spectra at the mid-point
       Bi = cmul(Bi, eb);
       if (obs) {
-        const double wgt = (kk == 0 || 2 * kk == N) ? 1.0 : 2.0;  // bins k and N - k
-        acc[1] += wgt * (double)(A.x * A.x + A.y * A.y + Bi.x * Bi.x + Bi.y * Bi.y);
-        if (kk == 0) add_x(c, 0.5 * (double)A.x, 0.5 * (double)Bi.y);
-        const double ux = wgt * (double)(A.x + Bi.y), uy = wgt * (double)(A.y - Bi.x);
+        const bool nyq = 2 * kk == N, self = kk == 0 || nyq;
+        const double wgt = self ? 1.0 : 2.0;  // bins k and N - k
+        const double ax = A.x, ay = A.y, bx = Bi.x, by = Bi.y;
+        acc[1] += wgt * (ax * ax + ay * ay + bx * bx + by * by);
+        if (kk == 0) add_x(c, 0.5 * ax, 0.5 * by);
+        const double ux = wgt * (ax + by), uy = self ? 0.0 : wgt * (ay - bx);
 #pragma unroll
         for (int q = 0; q < MAXO; ++q)
           if (q < a.Mp) {
-            const C gk = __ldg(G + (size_t)kk * MAXO + q);
-            acc[2 + MAXO + q] += ux * (double)gk.x + uy * (double)gk.y;
+            const double2 gk = __ldg(G + q * (N / 2) + (nyq ? 0 : kk));
+            acc[2 + MAXO + q] += ux * (nyq ? gk.y : gk.x) + uy * gk.y;
           }
       }
       if (!same) factors(a.tab2, a.g2, kk, c, ea, eb);
@@ -676,11 +679,13 @@ __global__ void __launch_bounds__(kGenThreads, gen_minb<Rl>()) gen_col_kernel(Pa
   gen_drain(z, N, lcp, store);
 }
 
-// Forward DFT of the p-observable weights of an even length P that is not a
-// power of two (see launch_pweight_dft): block (q, b) transforms vector q of
-// instance b in FP64, twiddles from sincospi of the exact ratio.
-template <typename Rl>
-__global__ void __launch_bounds__(kGenThreads) gen_pweight_kernel(const double* wp, long long wp_bs, int P, void* out,
+// Spectra of the p-observable weights for the fused generic pass: block (q, b)
+// transforms vector q of instance b in FP64, twiddles from sincospi of the exact
+// ratio.  They stay FP64 whatever the state's precision, so that an FP32 pass
+// weighs its spectra as exactly as it would its values: bins k < P/2 as
+// out[b][q][k], the real value at P/2 in the imaginary part of bin 0, which is
+// real too (the bytes of P complex FP32 entries a weight).
+__global__ void __launch_bounds__(kGenThreads) gen_pweight_kernel(const double* wp, long long wp_bs, int P, double2* out,
                                                                   long long out_bs, GenFactors g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* tw = reinterpret_cast<double2*>(smem_raw);
@@ -697,10 +702,10 @@ __global__ void __launch_bounds__(kGenThreads) gen_pweight_kernel(const double* 
   const double* w = wp + (size_t)b * wp_bs + (size_t)q * P;
   gen_fill(z, P, 0, [&](int p, int) { return make_double2(w[p], 0.0); });
   gen_fft<-1>(z, z2, P, g, 0, tw);
-  cplx_t<Rl>* o = reinterpret_cast<cplx_t<Rl>*>(out) + (size_t)b * out_bs + q;
-  for (int k = threadIdx.x; k < P; k += blockDim.x) {
+  double2* o = out + (size_t)b * out_bs + (size_t)q * (P / 2);
+  for (int k = threadIdx.x; k < P / 2; k += blockDim.x) {
     const double2 v = z[gen_slot<double2>(k)];
-    o[(size_t)k * 4] = mk<cplx_t<Rl>>((Rl)v.x, (Rl)v.y);
+    o[k] = k > 0 ? v : make_double2(v.x, z[gen_slot<double2>(P / 2)].x);
   }
 }
 
@@ -773,19 +778,13 @@ cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, in
 }
 
 cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
-                                   long long out_bs, int dtype, int dep, cudaStream_t st) {
+                                   long long out_bs, int dep, cudaStream_t st) {
   const GenFactors g = gen_factors(P, false);
-  const size_t smem = gen_smem<double2>(P, 0), smem_max = gen_smem<double2>(4096, 0);
-  static PerDeviceOnce attr[2];
-  if (dtype == FW_F32) {
-    cudaError_t e = set_smem_once(attr[0], gen_pweight_kernel<float>, smem_max);
-    if (e != cudaSuccess) return e;
-    return launch_dep(dep, gen_pweight_kernel<float>, dim3(Mp, nb), kGenThreads, smem, st, wp, wp_bs, P, out, out_bs, g);
-  } else {
-    cudaError_t e = set_smem_once(attr[1], gen_pweight_kernel<double>, smem_max);
-    if (e != cudaSuccess) return e;
-    return launch_dep(dep, gen_pweight_kernel<double>, dim3(Mp, nb), kGenThreads, smem, st, wp, wp_bs, P, out, out_bs, g);
-  }
+  static PerDeviceOnce attr;
+  cudaError_t e = set_smem_once(attr, gen_pweight_kernel, gen_smem<double2>(4096, 0));
+  if (e != cudaSuccess) return e;
+  return launch_dep(dep, gen_pweight_kernel, dim3(Mp, nb), kGenThreads, gen_smem<double2>(P, 0), st, wp, wp_bs, P, out,
+                    out_bs, g);
 }
 
 }  // namespace fw

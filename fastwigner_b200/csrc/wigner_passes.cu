@@ -320,7 +320,6 @@ __global__ void __launch_bounds__(256) pweight_dft_kernel(const double* wp, long
 
 cudaError_t launch_pweight_dft(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out, long long out_bs,
                                int dtype, int dep, cudaStream_t st) {
-  if (!is_pow2(P)) return launch_generic_pweight(wp, wp_bs, Mp, P, nb, out, out_bs, dtype, dep, st);
   const size_t smem = 2 * sizeof(double2) * (size_t)P;
   dim3 grid(Mp, nb);
   cudaError_t e;
