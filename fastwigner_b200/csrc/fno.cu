@@ -235,10 +235,12 @@ extern "C" int fw_fno_channel_sum(int Bn, int C, long long L, const float* X, fl
 // 0.07, near the time of reading both operands once).  A CTA stages 32 + 32 rows of
 // 128 pixels; each of its eight warps contracts 16 of them for the whole tile,
 // lane (rg, cg) owning rows rg + 8 i and columns cg + 4 j (128 FMAs per 12 vector
-// loads without bank conflicts).  A chain adds a few hundred pixels in FP32; warps
-// and CTAs are summed in FP64.
+// loads without bank conflicts).  A weight's chain adds at most 256 products in FP32
+// (kFlush stages); warps, flushes and CTAs are summed in FP64.  The bias sums are FP64
+// from the first addition, and stay so between CTAs as a high and a low float.
 namespace wgrad {
 constexpr int TP = 128, PITCH = TP + 4;
+constexpr int kFlush = 16;  // stages of 16 products a thread
 constexpr size_t SMEM = (size_t)2 * 32 * PITCH * 4;
 }  // namespace wgrad
 
@@ -256,13 +258,32 @@ __global__ void __launch_bounds__(256, 2) wgrad_kernel(int rows, int cols, long 
   const long long l0 = (long long)blockIdx.y * range, l1 = l0 + range < L ? l0 + range : L;
   const float* y = dY + (long long)blockIdx.z * sY;
   const float* x = X + (long long)blockIdx.z * sX;
-  float acc[4][8], bs[4];
+  const bool wb = bwork != nullptr && c0 == 0;
+  float acc[4][8];
+  double bs[4] = {0, 0, 0, 0}, ws[4] = {0, 0, 0, 0};  // bias sums of rows rg + 8 i; weights tid + 256 i of the tile
+  auto clear = [&] {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    bs[i] = 0.f;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  }
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  };
+  // the warps' chains through shared memory (8 x 1024 floats) into ws
+  auto flush = [&] {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sm[warp * 1024 + (rg + 8 * i) * 32 + cg + 4 * j] = acc[i][j];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      double s = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += (double)sm[w * 1024 + tid + 256 * i];
+      ws[i] += s;
+    }
+  };
+  clear();
   float4 ry[4], rx[4];
   auto fetch = [&](long long l) {  // warp w: rows w, w + 8, ...; lane: four pixels
     const bool in = l + 4 * lane < l1;
@@ -274,6 +295,7 @@ __global__ void __launch_bounds__(256, 2) wgrad_kernel(int rows, int cols, long 
     }
   };
   fetch(l0);
+  int stage = 0;
   for (long long l = l0; l < l1; l += TP) {
     __syncthreads();
 #pragma unroll
@@ -292,7 +314,6 @@ __global__ void __launch_bounds__(256, 2) wgrad_kernel(int rows, int cols, long 
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 a = *reinterpret_cast<const float4*>(Ys + (rg + 8 * i) * PITCH + p);
-        bs[i] += (a.x + a.y) + (a.z + a.w);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
@@ -302,32 +323,41 @@ __global__ void __launch_bounds__(256, 2) wgrad_kernel(int rows, int cols, long 
         }
       }
     }
+    if (wb)  // lane cg: a quarter of the warp's pixels
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(Ys + (rg + 8 * i) * PITCH + warp * 16 + 4 * cg);
+        bs[i] += ((double)a.x + (double)a.y) + ((double)a.z + (double)a.w);
+      }
+    if (++stage == kFlush && l + TP < l1) {
+      flush();
+      clear();
+      stage = 0;
+    }
   }
-  __syncthreads();
-  // the warps' tiles through shared memory (8 x 1024 floats), summed in FP64
+  flush();
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sm[warp * 1024 + (rg + 8 * i) * 32 + cg + 4 * j] = acc[i][j];
-  __syncthreads();
-  for (int e = tid; e < 1024; e += 256) {
-    const int r = r0 + (e >> 5), c = c0 + (e & 31);
-    double s = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) s += (double)sm[w * 1024 + e];
-    if (r < rows && c < cols) work[(long long)split * rows * cols + (long long)r * cols + c] = (float)s;
+  for (int i = 0; i < 4; ++i) {
+    const int e = tid + 256 * i, r = r0 + (e >> 5), c = c0 + (e & 31);
+    if (r < rows && c < cols) work[(long long)split * rows * cols + (long long)r * cols + c] = (float)ws[i];
   }
-  if (bwork != nullptr && c0 == 0) {
+  if (wb) {
+    double* bd = reinterpret_cast<double*>(sm);  // [warp][row]
     __syncthreads();
-    if (cg == 0)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sm[warp * 32 + rg + 8 * i] = bs[i];
+    for (int i = 0; i < 4; ++i) {
+      bs[i] += __shfl_xor_sync(0xffffffffu, bs[i], 1);
+      bs[i] += __shfl_xor_sync(0xffffffffu, bs[i], 2);
+      if (cg == 0) bd[warp * 32 + rg + 8 * i] = bs[i];
+    }
     __syncthreads();
     if (tid < 32 && r0 + tid < rows) {
       double s = 0;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) s += (double)sm[w * 32 + tid];
-      bwork[(long long)split * rows + r0 + tid] = (float)s;
+      for (int w = 0; w < 8; ++w) s += bd[w * 32 + tid];
+      float* o = bwork + 2 * ((long long)split * rows + r0 + tid);
+      o[0] = (float)s;
+      o[1] = (float)(s - (double)o[0]);
     }
   }
 }
@@ -339,7 +369,14 @@ __global__ void wgrad_sum_kernel(int Z, int E, int R, const float* __restrict__ 
   const bool w = e < E;
   double s = 0.0;
   if (e < E + R)
-    for (int z = threadIdx.y; z < Z; z += 8) s += w ? (double)work[(long long)z * E + e] : (double)bwork[(long long)z * R + e - E];
+    for (int z = threadIdx.y; z < Z; z += 8) {
+      if (w) {
+        s += (double)work[(long long)z * E + e];
+      } else {
+        const float* b = bwork + 2 * ((long long)z * R + e - E);
+        s += (double)b[0] + (double)b[1];
+      }
+    }
   __shared__ double red[8][33];
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
@@ -377,7 +414,7 @@ extern "C" int fw_fno_wgrad_bias_work(int rows, int cols, long long L, int batch
   int ns;
   long long range;
   wgrad_ranges(rows, cols, L, batch, &ns, &range);
-  *floats_out = (long long)batch * ns * rows * (cols + 1);
+  *floats_out = (long long)batch * ns * rows * (cols + 2);
   return FW_OK;
 }
 
@@ -392,7 +429,7 @@ extern "C" int fw_fno_wgrad_bias(int rows, int cols, long long L, const float* d
   long long range;
   wgrad_ranges(rows, cols, L, batch, &ns, &range);
   const long long z = (long long)batch * ns;
-  if (work_floats < z * rows * (cols + 1)) return fail(FW_EINVAL, "fw_fno_wgrad_bias: work buffer too small");
+  if (work_floats < z * rows * (cols + 2)) return fail(FW_EINVAL, "fw_fno_wgrad_bias: work buffer too small");
   float* bwork = bias != nullptr ? work + z * rows * cols : nullptr;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int nr = (rows + 31) / 32, nc = (cols + 31) / 32;
@@ -503,15 +540,16 @@ __global__ void __launch_bounds__(256, 2) project_bwd_kernel(long long L, int ba
       row8(x, ds);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float sc = 0.f, s2 = 0.f;
+        double sc = 0;
+        float s2 = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const float u = h[i][k] + b1[i];
           s2 = fmaf(gelu_tail(u), x[k], s2);
           h[i][k] = w2[i] * x[k] * gelu_d_tail(u);
-          sc += h[i][k];
+          sc += (double)h[i][k];
         }
-        gc[i] += (double)sc;
+        gc[i] += sc;
         g2[i] += (double)s2;
         float* r = dh + (4 * tj + i) * PX;
         *reinterpret_cast<float4*>(r + 4 * t8) = make_float4(h[i][0], h[i][1], h[i][2], h[i][3]);
