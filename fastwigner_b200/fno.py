@@ -370,6 +370,8 @@ class FNO2d:
         CS, Dpv, Dpiv, AA = self._grid(G0, G1)
         dev = self.device
         d_out = dout.contiguous().view(B, 1, G0, G1)
+        if d_out.data_ptr() % 16:  # (a view into a larger buffer; the kernels load four values at once)
+            d_out = d_out.clone()
         if self._fused_layers(G0, G1):
             dv = torch.empty((B, C, G0, G1), dtype=torch.float32, device=dev)
             o.project_bwd(L, B, c["vL"], P["Q1"], P["c1"], P["Q2"], d_out, dv, g["Q1"], g["c1"], g["Q2"], g["c2"])
