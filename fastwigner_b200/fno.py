@@ -70,7 +70,7 @@ class _Ops:
 
     def wgrad_bias(self, rows, cols, L, dY, X, batch, out, bias):
         """wgrad and csum in one pass: out, and bias[r] = sum_b sum_l dY[b][r][l]."""
-        if L % 4:  # (rows off 16 bytes)
+        if L % 4 or L > 1 << 30 or max(rows, cols) > 4096:  # (rows off 16 bytes; sizes past the kernel's)
             self.csum(batch, rows, L, dY, bias)
             return self.wgrad(rows, cols, L, dY, X, batch, out)
         n = ctypes.c_longlong(0)
@@ -300,7 +300,7 @@ class FNO2d:
         """Whether the fused layer kernels take this network and grid (fw_fno_layer):
         the surrogate's own width, modes and projection on any grid they hold."""
         return (self.C == 32 and self.mp == self.mx == 16 and self.proj == 128 and self.layers >= 1
-                and self.NP <= 14 and 32 <= G0 <= 1024 and G1 >= 32 and G1 % 4 == 0)
+                and self.NP <= 14 and 32 <= G0 <= 1024 and 32 <= G1 <= 65536 and G1 % 4 == 0)
 
     def _transposed(self, G0, G1):
         """The DFT matrices of _grid transposed, for the fused backward layers."""
