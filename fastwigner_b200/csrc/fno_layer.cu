@@ -603,9 +603,10 @@ __global__ void __launch_bounds__(128) fno_pidft_kernel(int G0, const float* __r
 
 // ---------------------------------------------------------------------------
 // Surrogate output: harmonic baseline + its peak x network, normalised.  The
-// baseline exp(-c H), H = p^2/2 + w^2 (x - x_e)^2/2, is a product of two
-// Gaussians, so its sum and its peak come from two vectors per sample; one
-// pass adds and sums (FP64), a second scales.
+// baseline exp(-c (H - min H)), H = p^2/2 + w^2 (x - x_e)^2/2 with its minimum over the
+// grid (a well centred far outside the box would underflow everywhere), is a
+// product of two Gaussians, so its sum and its peak come from two vectors per
+// sample; one pass adds and sums (FP64), a second scales.
 __device__ __forceinline__ double block_reduce(double v, double* red, bool max_) {
   for (int o = 16; o > 0; o >>= 1) {
     const double u = __shfl_xor_sync(0xffffffffu, v, o);
@@ -627,15 +628,23 @@ __global__ void __launch_bounds__(256) fno_thermal_kernel(int G0, int G1, const 
   const int b = blockIdx.y, tid = threadIdx.x;
   const double w = wc[2 * b], c = wc[2 * b + 1];
   const int per = (G0 + gridDim.x - 1) / gridDim.x, p0 = blockIdx.x * per, np = max(0, min(per, G0 - p0));
-  double sx = 0, mx = 0, sp = 0, mp = 0;
+  double sx = 0, mx = 0, sp = 0, mp = 0, ex = -INFINITY, ep = -INFINITY;  // ex, ep: less the minima of the two exponents
   for (int i = tid; i < G1; i += 256) {
-    const double d = w * (xs[i] - x_e), g = exp(-c * (0.5 * d * d));
+    const double d = w * (xs[i] - x_e), e = 0.5 * d * d;
+    gs[i] = e;
+    ex = fmax(ex, -e);
+  }
+  for (int i = tid; i < G0; i += 256) ep = fmax(ep, -0.5 * ps[i] * ps[i]);
+  ex = block_reduce(ex, red, true);
+  ep = block_reduce(ep, red, true);
+  for (int i = tid; i < G1; i += 256) {
+    const double g = exp(-c * (gs[i] + ex));
     gs[i] = g;
     sx += g;
     mx = fmax(mx, g);
   }
   for (int i = tid; i < G0; i += 256) {
-    const double g = exp(-c * (0.5 * ps[i] * ps[i]));
+    const double g = exp(-c * (0.5 * ps[i] * ps[i] + ep));
     if (i >= p0 && i < p0 + np) gs[G1 + i - p0] = g;
     sp += g;
     mp = fmax(mp, g);

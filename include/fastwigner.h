@@ -392,7 +392,7 @@ int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float*
 int fw_fno_pdft(int B, int G0, int G1, const float* fx, const float* Dpv, float* F2, void* stream);
 int fw_fno_pidft(int B, int G0, const float* O2, const float* Dpiv, float* gx, void* stream);
 /* out[b] (in: network output, out: thermal state) = B_b + max(B_b) out[b], scaled to sum out dxdp = 1, with B_b the
- * harmonic state exp(-c H), H = p^2/2 + w^2 (x - x_e)^2/2, of unit sum; wc: (w, c) per sample; work: 64 B doubles. */
+ * harmonic state exp(-c (H - min H)), H = p^2/2 + w^2 (x - x_e)^2/2, of unit sum; wc: (w, c) per sample; work: 64 B doubles. */
 int fw_fno_thermal(int B, int G0, int G1, const double* wc, const double* xs, const double* ps, double x_e, double dxdp,
                    float* out, double* work, void* stream);
 /* Backward of the projection (128 hidden, 32 channels) for dout = d(loss)/d(out): dV[b][32][L] and the gradients of Q1,
