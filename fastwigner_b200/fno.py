@@ -610,6 +610,12 @@ class BlochSurrogate:
         B = torch.exp(-c[:, None, None] * (Hh - Hh.amin(dim=(1, 2), keepdim=True)))
         return (B / B.sum(dim=(1, 2), keepdim=True)).float()
 
+    @staticmethod
+    def _wells(Ds, As, beta):
+        """(w, c) of baseline()'s exp(-c H_h) per well, FP64 from parameters of any type."""
+        w = np.asarray(As, dtype=np.float64) * np.sqrt(2.0 * np.asarray(Ds, dtype=np.float64))
+        return np.stack([w, (2.0 / w) * np.tanh(0.5 * np.asarray(beta, dtype=np.float64) * w)], axis=1)
+
     def _grid_device(self):
         """The full grid's x and p on the device (FP64)."""
         if getattr(self, "_xp_dev", None) is None:
@@ -665,8 +671,7 @@ class BlochSurrogate:
             out = self.net.forward(X, self.xs, self.ps, cache=False)
             if self.residual:
                 # baseline + its peak x network, normalised (the kernel evaluates baseline())
-                w = As[c0:c0 + chunk] * np.sqrt(2.0 * Ds[c0:c0 + chunk])
-                wc = np.stack([w, (2.0 / w) * np.tanh(0.5 * beta * w)], axis=1)
+                wc = self._wells(Ds[c0:c0 + chunk], As[c0:c0 + chunk], beta)
                 outs.append(self.net.ops.thermal(out, wc, *self._grid_device(), self.s.x_e, self.s.dX * self.s.dP))
                 continue
             outs.append(out / (out.double().sum(dim=(1, 2), keepdim=True) * self.s.dX * self.s.dP).float())
