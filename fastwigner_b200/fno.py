@@ -92,10 +92,10 @@ class _Ops:
                                     opt(fx), opt(out), opt(aux), opt(vcm), stream_handle()), "fw_fno_layer")
 
     def thermal(self, out, wc, xs, ps, x_e, dxdp):
-        """Thermal states from network outputs (in place), see fw_fno_thermal."""
+        """Thermal states from network outputs (in place), see fw_fno_thermal; wc, xs and
+        ps are FP64 on the device."""
         B, G0, G1 = out.shape
         dp = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
-        wc = torch.tensor(np.ascontiguousarray(wc, dtype=np.float64), device=out.device)
         work = torch.empty(64 * B, dtype=torch.float64, device=out.device)
         check(self.lib.fw_fno_thermal(B, G0, G1, dp(wc), dp(xs), dp(ps), float(x_e), float(dxdp), _p(out), dp(work),
                                       stream_handle()), "fw_fno_thermal")
@@ -616,11 +616,10 @@ class BlochSurrogate:
         w = np.asarray(As, dtype=np.float64) * np.sqrt(2.0 * np.asarray(Ds, dtype=np.float64))
         return np.stack([w, (2.0 / w) * np.tanh(0.5 * np.asarray(beta, dtype=np.float64) * w)], axis=1)
 
-    def _grid_device(self):
-        """The full grid's x and p on the device (FP64)."""
-        if getattr(self, "_xp_dev", None) is None:
-            self._xp_dev = tuple(t.to(self.net.device, torch.float64).contiguous() for t in self._xp_full)
-        return self._xp_dev
+    def _thermal_kernel(self):
+        """Whether fw_fno_thermal evaluates this object's baseline(): its own method, on a
+        grid whose row the kernel holds."""
+        return getattr(self.baseline, "__func__", None) is _BASELINE and self.s.G <= 16384
 
     def train(self, P, S, epochs=20, batch=16, lr=2e-3, rng=None, log=None, group=None):
         """P: (N, 3) raw (D, a, beta); S: (N, g, g) states (normalised to unit sum).
@@ -664,16 +663,24 @@ class BlochSurrogate:
         """Surrogate thermal Wigner functions on the full grid for instances
         (Ds, As) at one beta, each normalised to sum W dXdP = 1; (n, G, G)."""
         Ds, As = np.atleast_1d(Ds), np.atleast_1d(As)
-        outs = []
+        Ps = []
         for c0 in range(0, len(Ds), chunk):
-            X = normalise_params(np.stack([Ds[c0:c0 + chunk], As[c0:c0 + chunk],
-                                           np.full(len(Ds[c0:c0 + chunk]), beta)], axis=1))
-            out = self.net.forward(X, self.xs, self.ps, cache=False)
-            if self.residual:
-                # baseline + its peak x network, normalised (the kernel evaluates baseline())
-                wc = self._wells(Ds[c0:c0 + chunk], As[c0:c0 + chunk], beta)
-                outs.append(self.net.ops.thermal(out, wc, *self._grid_device(), self.s.x_e, self.s.dX * self.s.dP))
+            D = Ds[c0:c0 + chunk]
+            Ps.append(np.stack([D, As[c0:c0 + chunk], np.full(len(D), beta)], axis=1))
+        outs = []
+        kernel = self.residual and self._thermal_kernel()
+        if kernel:  # well parameters and axes in one upload
+            wells = [torch.from_numpy(self._wells(*P.T)).reshape(-1) for P in Ps]
+            axes = [t.to("cpu", torch.float64) for t in self._xp_full]
+            *wells, x, p = torch.cat(wells + axes).to(self.net.device).split([len(t) for t in wells + axes])
+        for k, P in enumerate(Ps):
+            out = self.net.forward(normalise_params(P), self.xs, self.ps, cache=False)
+            if kernel:  # baseline + its peak x network, normalised
+                outs.append(self.net.ops.thermal(out, wells[k], x, p, self.s.x_e, self.s.dX * self.s.dP))
                 continue
+            if self.residual:
+                B = self.baseline(P)
+                out = B + B.amax(dim=(1, 2), keepdim=True) * out
             outs.append(out / (out.double().sum(dim=(1, 2), keepdim=True) * self.s.dX * self.s.dP).float())
         return torch.cat(outs)
 
@@ -704,3 +711,6 @@ class BlochSurrogate:
         n = int(round(beta / self.s.dbeta))
         bb.run(n)
         return bb.W, n
+
+
+_BASELINE = BlochSurrogate.baseline  # what fw_fno_thermal evaluates
