@@ -744,6 +744,7 @@ extern "C" int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, c
 extern "C" int fw_fno_pdft(int B, int G0, int G1, const float* fx, const float* Dpv, float* F2, void* stream) {
   if (int rc = check_dims(B, G0, G1, "fw_fno_pdft")) return rc;
   if (fx == nullptr || Dpv == nullptr || F2 == nullptr) return fail(FW_EINVAL, "fw_fno_pdft: NULL argument");
+  if (((uintptr_t)Dpv & 7u) != 0) return fail(FW_EINVAL, "fw_fno_pdft: Dpv must start on 8 bytes");
   const size_t tab = (size_t)((G0 + kPdftSplit - 1) / kPdftSplit) * 2 * LM * 4, red = 4 * LM * 16 * 16;
   const size_t smem = tab > red ? tab : red;  // at most 34 KiB (G0 = 1024)
   const int tiles = (G1 + LX - 1) / LX;

@@ -388,7 +388,8 @@ int fw_fno_layer(int mode, int B, int G0, int G1, const float* vin, const float*
                  const float* Q1, const float* c1, const float* Q2, const float* c2, float* vout, float* fx, float* out,
                  const float* aux, float* vcm, void* stream);
 /* F2[b][c][2][32 x 16] = p-transform of fx (tiles summed); gx[b][p][c][32 parts] (swizzled rows) = inverse
- * p-transform of O2.  Dpv, Dpiv: the interleaved DFT matrices (64 x 2 G0, 2 G0 x 64). */
+ * p-transform of O2.  Dpv, Dpiv: the interleaved DFT matrices (64 x 2 G0, on 8 bytes, and
+ * 2 G0 x 64). */
 int fw_fno_pdft(int B, int G0, int G1, const float* fx, const float* Dpv, float* F2, void* stream);
 int fw_fno_pidft(int B, int G0, const float* O2, const float* Dpiv, float* gx, void* stream);
 /* out[b] (in: network output, out: thermal state) = B_b + max(B_b) out[b], scaled to sum out dxdp = 1, with B_b the
