@@ -43,34 +43,26 @@ template <int N> struct TabBox {
   static_assert(ROWS <= 256, "table box too tall");
 };
 
-// Launch shapes of the persistent column pass.  MINB CTAs of CP*T threads per
-// SM.  BMAJOR: work items instance-major (consecutive items of a CTA are
-// neighbouring column tiles of one instance, so a tile whose rows are narrower
-// than a 64-byte DRAM line finds the rest of the line in L2; the table tile is
-// fetched for every item) instead of column-tile major (consecutive items share
-// the table tile).  PSUM_ALIAS: the per-bin p-weight sums live in the table
-// tile's buffer once the mid-point has read the table (only with a table fetch
-// per item).
+// Launch shapes of the persistent column pass: MINB CTAs of CP*T threads per SM.
+// Work items are column-tile major, so that consecutive items of a CTA share the
+// table tile.
 template <int N> struct ColpShape;
-// 1024: one CTA of 16 warps per SM, eight column pairs (64-byte state rows),
-// column-tile-major items so a shared table tile is fetched once per column
-// tile a CTA visits.  (Four pairs at two CTAs per SM, instance-major with a
-// table fetch per item and the sums in the table buffer, measured 0.330 vs
-// 0.315 ms per 64 x 1024^2 launch.)
+// 1024: one CTA of 16 warps per SM, eight column pairs (64-byte state rows).
+// (Four pairs at two CTAs per SM, instance-major with a table fetch per item and
+// the per-bin sums in the table's buffer, measured 0.330 vs 0.315 ms per
+// 64 x 1024^2 launch.)
 template <> struct ColpShape<1024> {
   static constexpr int T = 64, CP = 8, MINB = 1;
-  static constexpr bool BMAJOR = false, PSUM_ALIAS = false;
 };
 
-template <int N, int T, int CP, bool PSUM_ALIAS> struct ColpLayout {
+template <int N, int T, int CP> struct ColpLayout {
   static constexpr int WROWB = 2 * CP;                        // floats per state-tile row
   static constexpr size_t W_FLOATS = (size_t)N * WROWB;
   static constexpr size_t T_FLOATS = (size_t)TabBox<N>::NL * TabBox<N>::ROWS * 4 * CP;  // complex tables
   static constexpr size_t EX_FLOATS = col_ex_reals<float, N, T, CP>();
-  static constexpr size_t PSUM_FLOATS = PSUM_ALIAS ? 0 : (size_t)2 * N;
+  static constexpr size_t PSUM_FLOATS = (size_t)2 * N;
   // + twiddles, + 128 bytes to align the base of the buffers
   static constexpr size_t BYTES = (W_FLOATS + T_FLOATS + EX_FLOATS + PSUM_FLOATS) * 4 + (size_t)N * 8 + 128;
-  static_assert(!PSUM_ALIAS || T_FLOATS >= (size_t)2 * N, "psum must fit in the table buffer");
   // every bulk-tensor destination on 128 bytes: the state boxes, the table
   // buffer and each table box (complex and real tables)
   static_assert((W_FLOATS * 4) % 128 == 0 && ((size_t)(N < 256 ? N : 256) * WROWB * 4) % 128 == 0,
@@ -156,12 +148,12 @@ struct ColpCtl {
   int tab_inst;  // phase tables per instance (1) or one for the batch (0)
 };
 
-template <int N, int T, int CP, int MINB, bool BMAJOR, bool PSUM_ALIAS, bool FUSED, bool OBS>
+template <int N, int T, int CP, int MINB, bool FUSED, bool OBS>
 __global__ void __launch_bounds__(CP* T, MINB)
     col_persist_kernel(const __grid_constant__ CUtensorMap mW, const __grid_constant__ CUtensorMap mT, PassArgs a,
                        ColpCtl ctl) {
   using C = float2;
-  using L = ColpLayout<N, T, CP, PSUM_ALIAS>;
+  using L = ColpLayout<N, T, CP>;
   constexpr int RV = N / T;
   constexpr int NTHR = CP * T;
   constexpr int WBOX = N < 256 ? N : 256;  // state rows per bulk copy
@@ -176,7 +168,7 @@ __global__ void __launch_bounds__(CP* T, MINB)
   float* Ts = Ws + L::W_FLOATS;
   float* exb = Ts + L::T_FLOATS;
   C* tw = reinterpret_cast<C*>(exb + L::EX_FLOATS);
-  C* psum = PSUM_ALIAS ? reinterpret_cast<C*>(Ts) : tw + N;
+  C* psum = tw + N;
 
   const int n_items = a.batch * ctl.ntiles;
   const int first = (int)((long long)blockIdx.x * n_items / gridDim.x);
@@ -187,11 +179,10 @@ __global__ void __launch_bounds__(CP* T, MINB)
   constexpr int tab_rowf = 4 * CP;  // floats per table-tile row (complex tables)
   const uint32_t w_bytes = (uint32_t)(L::W_FLOATS * 4);
   const uint32_t t_bytes = (uint32_t)(TabBox<N>::NL * TabBox<N>::ROWS * tab_rowf * 4);
-  auto item_t = [&](int it) { return BMAJOR ? it % ctl.ntiles : it / a.batch; };
-  auto item_b = [&](int it) { return BMAJOR ? it / ctl.ntiles : it % a.batch; };
-  // key of the table tile an item reads; with the p-weight sums in the table
-  // buffer every item fetches its tile
-  auto tab_key = [&](int it) { return (ctl.tab_inst || PSUM_ALIAS) ? it : item_t(it) * a.batch; };
+  auto item_t = [&](int it) { return it / a.batch; };
+  auto item_b = [&](int it) { return it % a.batch; };
+  // key of the table tile an item reads
+  auto tab_key = [&](int it) { return ctl.tab_inst ? it : item_t(it) * a.batch; };
   auto issue_w = [&](int it) {
     mbar_arrive_expect_tx(&bars[0], w_bytes);
 #pragma unroll
@@ -273,10 +264,8 @@ __global__ void __launch_bounds__(CP* T, MINB)
     fused_mid_staged<N, T, RV, CP, FUSED, OBS>(a, b, v, j, ex, c, Ts, psum, o, sc);  // ends with a CTA barrier
     const int xa = tile * 2 * CP + 2 * c;
     if (OBS) mid_store<float, N, CP, NTHR>(a, b, tile, ctl.ntiles, o, xa, ored);
-    // the next item's table tile (the p-weight sums in the table buffer have
-    // been read before mid_store's barrier)
+    // the next item's table tile
     t_pending = it + 1 < last && tab_key(it + 1) != tab_key(it);
-    if (PSUM_ALIAS && !OBS) __syncthreads();  // no mid_store barrier to lean on
     if (tid == 0 && t_pending) issue_t(it + 1);
     // ---- inverse transform and store
     fft<N, T, RV, +1, C, EXT>(v, j, ex, tw);
@@ -331,7 +320,7 @@ template <int N>
 cudaError_t launch_colp_cfg(const PassArgs& a, cudaStream_t st, int* nparts) {
   using S = ColpShape<N>;
   constexpr int T = S::T, CP = S::CP;
-  using L = ColpLayout<N, T, CP, S::PSUM_ALIAS>;
+  using L = ColpLayout<N, T, CP>;
   const int P = a.P, X = a.X;
   const int ntiles = X / (2 * CP);
   const int tab_rowf = (a.tab_real ? 2 : 4) * CP;
@@ -350,10 +339,10 @@ cudaError_t launch_colp_cfg(const PassArgs& a, cudaStream_t st, int* nparts) {
                  (uint32_t)TabBox<N>::ROWS, CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
     return cudaErrorInvalidValue;
   const bool obs = a.part_out != nullptr;
-  auto kern = a.fuse_mid ? (obs ? col_persist_kernel<N, T, CP, S::MINB, S::BMAJOR, S::PSUM_ALIAS, true, true>
-                                : col_persist_kernel<N, T, CP, S::MINB, S::BMAJOR, S::PSUM_ALIAS, true, false>)
-                         : (obs ? col_persist_kernel<N, T, CP, S::MINB, S::BMAJOR, S::PSUM_ALIAS, false, true>
-                                : col_persist_kernel<N, T, CP, S::MINB, S::BMAJOR, S::PSUM_ALIAS, false, false>);
+  auto kern = a.fuse_mid ? (obs ? col_persist_kernel<N, T, CP, S::MINB, true, true>
+                                : col_persist_kernel<N, T, CP, S::MINB, true, false>)
+                         : (obs ? col_persist_kernel<N, T, CP, S::MINB, false, true>
+                                : col_persist_kernel<N, T, CP, S::MINB, false, false>);
   static PerDeviceOnce attr[4];
   cudaError_t e = set_smem_once(attr[(a.fuse_mid ? 2 : 0) + (obs ? 1 : 0)], kern, L::BYTES);
   if (e != cudaSuccess) return e;
