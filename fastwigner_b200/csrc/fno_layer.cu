@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
   extern __shared__ __align__(128) unsigned char sm_dyn[];
   __shared__ __align__(8) uint64_t bars[2][5];  // per slot: [0], [1] loads of v into buffer 0, 1; [2] D1 done; [3] D2 / hidden done; [4] load of G
   __shared__ uint32_t tmem_base;
-  __shared__ int abort_flag[2];
   __shared__ float s_bias[LC], s_c1[PROJ], s_q2[PROJ], s_row[2][LC];
   unsigned char* sm = sm_dyn + ((1024u - (smem_u32(sm_dyn) & 1023u)) & 1023u);
   const int tid = threadIdx.x, st = tid & 127, lane = tid & 31;
@@ -139,7 +138,6 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
     for (int s = 0; s < 2; ++s)
       for (int i = 0; i < 5; ++i) mbar_init(&bars[s][i], 1);
     mbar_fence_init();
-    abort_flag[0] = abort_flag[1] = 0;
   }
   float* AAh = reinterpret_cast<float*>(sm + S_AAH);
   float* AAl = reinterpret_cast<float*>(sm + S_AAL);
@@ -208,6 +206,24 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
     return ((size_t)b * LC * a.G0 + (r - b * a.G0)) * a.G1 + x0 + st;
   };
   auto slot_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory"); };
+  // a wait of this thread ran out.  The slot's threads decide on it together, at
+  // their barrier: a flag in memory, set by a later wait while a slower thread still
+  // reads it for the earlier one, would part them
+  bool bad = false;
+  auto slot_any = [&](bool v) {  // slot_sync that returns whether any thread of the slot brought v
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "r"(1 + slot)
+        : "memory");
+    return r != 0;
+  };
   auto load_v = [&](int r, int buf) {  // one thread of the slot
     mbar_arrive_expect_tx(&bar[buf], vbytes);
     bulk_load(mine + T_V + buf * 16384, a.vin + ((size_t)r * a.G1 + x0) * LC, vbytes, &bar[buf]);
@@ -230,7 +246,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
   int prev = 0;
   // D2 (or the hidden layer) complete: its operands' buffers may be written again
   auto wait_d2 = [&] {
-    if (!mbar_wait_bounded(&bar[3], ph2, kLayerPolls)) abort_flag[slot] = 1;
+    if (!mbar_wait_bounded(&bar[3], ph2, kLayerPolls)) bad = true;
     ph2 ^= 1u;
     tc_fence_after();
   };
@@ -272,9 +288,9 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
     d2_pending = false;
     float v[LC];
     if (MODE != LAYER_LIFT) {
-      if (!mbar_wait_bounded(&bar[buf], (ph_ld >> buf) & 1u, kLayerPolls)) abort_flag[slot] = 1;
+      if (!mbar_wait_bounded(&bar[buf], (ph_ld >> buf) & 1u, kLayerPolls)) bad = true;
       ph_ld ^= 1u << buf;
-      if (!mbar_wait_bounded(&bar[4], ph_g, kLayerPolls)) abort_flag[slot] = 1;
+      if (!mbar_wait_bounded(&bar[4], ph_g, kLayerPolls)) bad = true;
       ph_g ^= 1u;
       // split in place: high parts stay, low parts beside them
       float4 w[10];  // all loads first
@@ -293,9 +309,9 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
       }
       proxy_fence_smem();
       tc_fence_before();
-      slot_sync();
+      ok = !slot_any(bad);
       tc_fence_after();
-      if (abort_flag[slot]) { ok = false; break; }
+      if (!ok) break;
       const int nr = r + stride;
       if (warp == 0 && elect_lane()) {
         const uint32_t id2 = instr_desc(2 * LC), id = instr_desc(LC), aV = smem_u32(V);
@@ -314,7 +330,7 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
         }
       }
       if (MODE == LAYER_MID && d2_prev) store_d2();  // while D1 is computed
-      if (!mbar_wait_bounded(&bar[2], ph1, kLayerPolls)) abort_flag[slot] = 1;
+      if (!mbar_wait_bounded(&bar[2], ph1, kLayerPolls)) bad = true;
       ph1 ^= 1u;
       tc_fence_after();
       if (nr < a.rows && warp == 0 && elect_lane()) load_g(nr);
@@ -399,9 +415,9 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
     }
     proxy_fence_smem();
     tc_fence_before();
-    slot_sync();
+    ok = !slot_any(bad);
     tc_fence_after();
-    if (abort_flag[slot]) { ok = false; break; }
+    if (!ok) break;
     if (warp == 0 && elect_lane()) {
       if (MODE != LAYER_LAST) {
         const uint32_t id = (instr_desc(2 * LC) & ~(0x1Fu << 24)) | (4u << 24);  // M = 64
@@ -445,9 +461,10 @@ __global__ void __launch_bounds__(256, 1) fno_layer_kernel(LayerArgs a) {
     store_d2();
     d2_pending = false;
   }
-  if (!ok || abort_flag[slot]) {
-    if (warp == 0 && elect_lane()) {
-      atomicCAS(a.status, 0, FW_FNO_TIMEOUT);
+  if (bad) atomicCAS(a.status, 0, FW_FNO_TIMEOUT);
+  if (warp == 0) {
+    const bool drain = !ok || __any_sync(0xffffffffu, bad);
+    if (drain && elect_lane()) {
       // products and copies still in flight: once more, bounded, before the buffers are released
       mbar_wait_bounded(&bar[2], ph1, kLayerPolls >> 8);
       if (d2_pending) mbar_wait_bounded(&bar[3], ph2, kLayerPolls >> 8);
