@@ -24,7 +24,7 @@ int cuda_fail(cudaError_t e, const char* where) {
 
 // exp(-2 pi i k / N), k < N, computed in FP64 with the angle reduced exactly
 // through integer arithmetic on k (so the table is accurate to FP64 rounding).
-static std::vector<double> twiddles(int n) {
+std::vector<double> twiddles(int n) {
   std::vector<double> t(2 * (size_t)n);
   for (int k = 0; k < n; ++k) {
     const double a = -2.0 * M_PI * (double)k / (double)n;
@@ -34,27 +34,30 @@ static std::vector<double> twiddles(int n) {
   return t;
 }
 
-// Stage-layout twiddle table of an n-point transform with rv values per
-// thread (fft.cuh, stage_off): the entries of twiddles(n) at k = bm r n/(ns R),
-// computed by the same expression, so both tables hold identical values.
-static std::vector<double> stage_twiddles(int n, int rv) {
-  std::vector<double> t;
+// Appends to t = twiddles(n) the stage-layout table of an n-point transform with
+// rv values per thread (fft.cuh, stage_off): its entries at k = bm r n/(ns R).
+void stage_twiddles(std::vector<double>& t, int n, int rv) {
+  const size_t at = t.size();
+  t.reserve(2 * at);
   for (int ns = rv; ns < n; ns *= rv) {
     const int R = n / ns >= rv ? rv : n / ns;
     const int s = n / (ns * R);
     for (int r = 1; r < R; ++r)
       for (int bm = 0; bm < ns; ++bm) {
-        const double a = -2.0 * M_PI * (double)(bm * r * s) / (double)n;
-        t.push_back(cos(a));
-        t.push_back(sin(a));
+        const size_t k = (size_t)bm * r * s;
+        t.push_back(t[2 * k]);
+        t.push_back(t[2 * k + 1]);
       }
   }
-  if (t.empty()) t.assign(2, 0.0);
-  return t;
+  if (t.size() == at) t.insert(t.end(), 2, 0.0);
 }
 
-int upload_twiddles(int n, int dtype, void** dev, int rv) {
-  std::vector<double> t = rv > 0 ? stage_twiddles(n, rv) : twiddles(n);
+static int upload_twiddles(int n, int dtype, void** dev, int rv) {
+  std::vector<double> t = twiddles(n);
+  if (rv > 0) {
+    stage_twiddles(t, n, rv);
+    t.erase(t.begin(), t.begin() + 2 * (size_t)n);
+  }
   cudaError_t e;
   if (dtype == FW_F64) {
     e = cudaMalloc(dev, t.size() * sizeof(double));

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <mutex>
 #include <string>
+#include <vector>
 #include "../../include/fastwigner.h"
 
 namespace fw {
@@ -80,8 +81,9 @@ cudaError_t launch_generic_col(const PassArgs& a, int dtype, cudaStream_t st, in
 cudaError_t launch_generic_pweight(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out,
                                    long long out_bs, int dep, cudaStream_t st);
 
-// device table exp(-2 pi i k/n), k < n, or (rv > 0) its stage layout for rv values per thread
-int upload_twiddles(int n, int dtype, void** dev, int rv);
+// exp(-2 pi i k/n), k < n, and its stage layout for rv values per thread appended
+std::vector<double> twiddles(int n);
+void stage_twiddles(std::vector<double>& t, int n, int rv);
 // 1 unless `st` is being captured
 int dep_launches(cudaStream_t st);
 
