@@ -321,18 +321,14 @@ __global__ void __launch_bounds__(256) pweight_dft_kernel(const double* wp, long
 cudaError_t launch_pweight_dft(const double* wp, long long wp_bs, int Mp, int P, int nb, void* out, long long out_bs,
                                int dtype, int dep, cudaStream_t st) {
   const size_t smem = 2 * sizeof(double2) * (size_t)P;
-  dim3 grid(Mp, nb);
-  cudaError_t e;
-  if (dtype == FW_F32) {
-    e = cudaFuncSetAttribute(pweight_dft_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = launch_dep(dep, pweight_dft_kernel<float>, grid, 256, smem, st, wp, wp_bs, P, out, out_bs);
-  } else {
-    e = cudaFuncSetAttribute(pweight_dft_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = launch_dep(dep, pweight_dft_kernel<double>, grid, 256, smem, st, wp, wp_bs, P, out, out_bs);
-  }
-  return e;
+  // the attribute is the largest size any launch may use, set once: set to each
+  // call's size, another thread's smaller one could come before this launch
+  const size_t smem_max = 2 * sizeof(double2) * 4096;
+  static PerDeviceOnce attr[2];
+  auto kern = dtype == FW_F32 ? pweight_dft_kernel<float> : pweight_dft_kernel<double>;
+  cudaError_t e = set_smem_once(attr[dtype == FW_F32 ? 0 : 1], kern, smem_max);
+  if (e != cudaSuccess) return e;
+  return launch_dep(dep, kern, dim3(Mp, nb), 256, smem, st, wp, wp_bs, P, out, out_bs);
 }
 
 }  // namespace fw
