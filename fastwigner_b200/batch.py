@@ -217,9 +217,10 @@ class WignerMoyalUnevenBatch:
     * variants 0 .. GROUPED-1: one persistent cooperative launch per
       ``propagate`` call over every instance, in one of the launch shapes;
     * GROUPED: instances of one (P, X, dX dP) share one state buffer, one
-      table buffer and one plan of the single-shape path, and the groups run
-      one after another (the persistent pass kernels where a group is large
-      enough, the regular ones otherwise).
+      table buffer and one plan of the single-shape path (the persistent pass
+      kernels where a group is large enough, the regular ones otherwise); the
+      groups run one after another when launched directly, in parallel branches
+      when replayed as a graph.
 
     ``specs``: one dict per instance with X_gridDIM, P_gridDIM, X_amplitude,
     P_amplitude, V (callable of x), K (callable of p).  ``variant`` None picks

@@ -22,7 +22,7 @@ seeds follow the workloads the propagators are specified on:
   a ~ U(0.02, 0.1), b ~ U(0.5, 2), amplitude 10, dt 0.005, replayed as a
   CUDA graph; the autotuner picks between the launch shapes of the persistent
   cooperative kernel (one launch per call) and the grouped mode (one plan per
-  grid shape, the groups one after another in one graph).
+  grid shape, the groups in parallel branches of one graph).
 * ``strong_field`` -- velocity-gauge laser-driven soft-core atom with
   random-collision dephasing: V0 = -1/sqrt(x^2 + 1), E(t) = E0 sin^2(pi t/T)
   sin(w t), E0 ~ U(0.01, 0.1), w = 0.057, T = 8 cycles, x: 2048 points

@@ -41,7 +41,8 @@ constexpr size_t kGenSmem32 = (size_t)56 << 10, kGenSmem64 = (size_t)110 << 10;
 // their own.  The rounding of such long FP32 sums is the same function of the
 // data in every step, so it adds up: at P = 1198 (prime 599), 1150 points and
 // 20 steps the other order alone moves the kinetic-energy sums by 6e-5 of the
-// record, at primes up to 59 by less than 1e-5.  FP64 has no such limit.
+// record, at primes up to 59 by less than 1e-5.  The line keeps results where they
+// were; which order is nearer to 64 bits was not measured.  FP64 has no such limit.
 constexpr int kGenSequentialAbove = 64;
 
 // Stage s: radix ra * rb (rb = 1: one factor) on top of transforms of length
